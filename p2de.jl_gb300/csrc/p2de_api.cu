@@ -242,6 +242,8 @@ struct p2de_solver {
   StageGeometry geo{};
   bool mixed = false;
   bool axis_aligned = true;
+  bool own_boundaries = true;  // every face with a boundary code is its own exterior face
+  bool flux = false;           // stage kernels in flux form
   // device memory
   double *Uq = nullptr, *resW = nullptr, *rhsL = nullptr, *rhsH = nullptr, *rhsU = nullptr;
   double *rhsxyL = nullptr, *rhsxyH = nullptr, *BFL = nullptr, *BFH = nullptr;
@@ -341,6 +343,8 @@ int flags_for(const p2de_solver* s, int nstage, bool update, bool debug) {
     f |= F_GAUSS;
     if (s->prm.entropyproj_limiter == P2DE_ENTROPYPROJ_NODEWISE_SCALED_EXTRAPOLATION) f |= F_EPROJ;
   }
+  if (flux_form(f, s->prm.N, s->prm.ZEROTOL, s->own_boundaries,
+                s->prm.precision == P2DE_PRECISION_MIXED)) f |= F_FLUX;
   if (update) f |= F_UPDATE;
   if (debug) f |= F_WRITE_DEBUG;
   return f;
@@ -607,6 +611,13 @@ int p2de_initialize_DG(const p2de_param* prm, const p2de_mesh* mesh, int device,
       return bail(P2DE_ERR_INVALID_ARGUMENT);
     }
   }
+  s->own_boundaries = own_faces(mesh->mapI, mesh->nI, mesh->mapP) && own_faces(mesh->mapO, mesh->nO, mesh->mapP) &&
+                      own_faces(mesh->mapW, mesh->nW, mesh->mapP) && own_faces(mesh->mapS, mesh->nS, mesh->mapP);
+  s->flux = flags_for(s, 2, false, false) & F_FLUX;
+  if (s->flux) {  // its own shared-memory layout
+    s->geo.elems_per_block = s->geo.elems_per_block_flux;
+    s->geo.elems_per_block_max = s->geo.elems_per_block_max_flux;
+  }
 #define DA(ptr, cnt)                                                                     \
   do {                                                                                   \
     cudaError_t ee = dalloc(s, &(ptr), (cnt));                                           \
@@ -664,6 +675,7 @@ int p2de_initialize_DG(const p2de_param* prm, const p2de_mesh* mesh, int device,
   StageArgs& a = s->base;
   a.K = s->K;
   a.epb = s->geo.elems_per_block;
+  if (s->flux) a.threads = flux_threads(s->K, a.epb);
   a.ops = table_of(s);
   a.Uq = s->Uq;
   a.resW = s->resW;
@@ -681,8 +693,7 @@ int p2de_initialize_DG(const p2de_param* prm, const p2de_mesh* mesh, int device,
     a.shock_post[c] = mesh->shock_post[c];
     a.shock_pre[c] = mesh->shock_pre[c];
   }
-  a.gamma = prm->gamma;
-  a.gm1 = prm->gamma - 1.0;
+  set_gas(a, prm->gamma);
   a.CFL = prm->CFL;
   a.dt0 = prm->dt0;
   a.T = prm->T;
@@ -801,6 +812,26 @@ int p2de_get_field(p2de_solver* s, int32_t field, int32_t nstage, double* out) {
       CK(cudaStreamSynchronize(s->stream));
       const int hl = field == P2DE_FIELD_F_BAR_H ? 0 : 1;
       const int nc = s->kpp ? 1 : 4;  // KPP: the scalar in component 0
+      if (s->flux) {
+        // flux form keeps [d][f_H - f_L, f_L][face][c] in units of -g w (p2de_flux.cuh)
+        double r[kMaxN1D], w[kMaxN1D], D[kMaxN1D * kMaxN1D];
+        gll_rule(s->N, r, w, D);
+        std::vector<double> geom(5 * K);
+        CK(cudaMemcpyAsync(geom.data(), s->geom, sizeof(double) * geom.size(), cudaMemcpyDeviceToHost, s->stream));
+        CK(cudaStreamSynchronize(s->stream));
+        const size_t n = (size_t)s->N1D;
+        for (size_t d = 0; d < 2; ++d)
+          for (size_t k = 0; k < K; ++k)
+            for (size_t f = 0; f < nsf; ++f) {
+              const double unit = -(geom[5 * k + (d ? 4 : 1)] * w[d ? f % n : f / (n + 1)]);
+              for (int c = 0; c < 4; ++c) {
+                const double fL = fb[16 * nsf * k + ((d * 2 + 1) * nsf + f) * 4 + c];
+                const double df = fb[16 * nsf * k + (d * 2 * nsf + f) * 4 + c];
+                out[4 * (f + nsf * (k + K * d)) + c] = unit * (hl == 0 ? fL + df : fL);
+              }
+            }
+        return P2DE_OK;
+      }
       for (size_t d = 0; d < 2; ++d)
         for (size_t k = 0; k < K; ++k)
           for (size_t f = 0; f < nsf; ++f)
@@ -1141,7 +1172,7 @@ int p2de_autotune(p2de_solver* s, int32_t* best_epb, double* best_ms) {
     if (e <= emax && std::find(cand.begin(), cand.end(), e) == cand.end()) cand.push_back(e);
   // the lines-per-warp layout differs from the flat one on axis-aligned LGL elements only
   std::vector<int> layouts{P2DE_LAYOUT_FLAT};
-  if (!s->gauss && !s->kpp && (flags_for(s, 2, false, false) & F_AXIS_ALIGNED))
+  if (!s->gauss && !s->kpp && !s->flux && (flags_for(s, 2, false, false) & F_AXIS_ALIGNED))
     layouts.push_back(P2DE_LAYOUT_LINES_PER_WARP);
   int best_layout = s->base.layout;
   int best_threads = s->base.threads > 0 ? s->base.threads : s->geo.threads;

@@ -32,7 +32,8 @@ enum : int {
   F_GAUSS = 1 << 18,        // GaussCollocation: projected face states, face pairs, Vf lift
   F_EPROJ = 1 << 19,        // NodewiseScaledExtrapolation: theta per face node
   F_KPP = 1 << 20,          // KPP{Dim2}: the scalar in component 0, the others 0
-  F_LFPROJ = 1 << 21        // LaxFriedrichsOnProjectedVal low-order flux: its CFL term
+  F_LFPROJ = 1 << 21,       // LaxFriedrichsOnProjectedVal low-order flux: its CFL term
+  F_FLUX = 1 << 22          // stage kernels in flux form (flux_form, p2de_flux.cuh)
 };
 // the modes whose branches only the EXT instantiation of stage kernel A compiles
 constexpr int kExtFlags = F_ZHANG_SHU | F_MIN_ENTROPY | F_RELAXED | F_GAUSS | F_EPROJ | F_KPP | F_LFPROJ;
@@ -94,7 +95,45 @@ struct StageArgs {
   double* ufproj;       // K x Nfp x 4: entropy-projected face states (GaussCollocation)
   double* theta;        // 3 stages x K x Nfp: entropy-projection limiting factors
   double eta;           // LimitingParameter eta (bounds of the projected face states)
+  // constants of the gas, formed once (set_gas): 1/(gamma-1), (gamma-1)/2, gamma (gamma-1)/4,
+  // and FP32 gamma, gamma-1, 2 (gamma-1)
+  double rgm1, hgm1, cws;
+  float gasf[3];
 };
+
+inline void set_gas(StageArgs& a, double gamma) {
+  a.gamma = gamma;
+  a.gm1 = gamma - 1.0;
+  a.rgm1 = 1.0 / a.gm1;
+  a.hgm1 = 0.5 * a.gm1;
+  a.cws = 0.25 * (gamma * a.gm1);
+  a.gasf[0] = (float)a.gamma;
+  a.gasf[1] = (float)a.gm1;
+  a.gasf[2] = (float)(2.0 * a.gm1);
+}
+
+// Whether every face node of a boundary list (1-based, as mapI, mapO, mapW, mapS) is its own
+// exterior face.
+inline bool own_faces(const int64_t* list, int64_t count, const int64_t* mapP) {
+  for (int64_t i = 0; i < count; ++i)
+    if (mapP[list[i] - 1] != list[i]) return false;
+  return true;
+}
+
+// Whether a solve's stage kernels run in flux form (p2de_flux.cuh): subcell-limited Euler on
+// axis-aligned LGL elements with the nodal low-order flux. own_boundaries: every face with a
+// boundary code is its own exterior face (mapP), as uniform meshes have it; the limited flux
+// there then needs no neighbour's factor. No low-order pair may have been dropped by ZEROTOL
+// (its entry is half the tangential weight, at least 1/(N (N+1))), since the form divides
+// the lines' common weight out. acc32: the FP32 two-point sums of mixed precision do not
+// telescope, and whether the difference they leave at an element face blends is decided by
+// the sign of FP64 rounding, so those solves keep the nodal form and its bits. Under the reference's reading of the bounds every interior
+// factor is 0, so a shock-capture cap acts only on the rounding of f_bar_H - f_bar_L at
+// element faces, which the flux form makes exactly 0: those solves keep the nodal form.
+inline bool flux_form(int flags, int N, double zerotol, bool own_boundaries, bool acc32) {
+  return (flags & F_AXIS_ALIGNED) && (flags & F_DO_LIMIT) && !(flags & (F_GAUSS | F_KPP | F_LFPROJ | F_ZHANG_SHU)) &&
+         !((flags & F_SHOCK) && (flags & F_REF_SEM)) && !acc32 && own_boundaries && zerotol < 0.999999 / ((double)N * (N + 1));
+}
 
 // StageArgs shock-capture constants of update_blending_factor! (shock_capture.jl:123-126)
 inline void set_shock_capture(StageArgs& a, int N, double sc_a, double sc_c) {

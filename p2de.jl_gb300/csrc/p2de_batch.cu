@@ -144,7 +144,7 @@ Layout layout_for(const p2de_param& p, int64_t nI, int64_t nS) {
 // The flags of a member as the one-solve path sets them for its stage kernels (without
 // the stage-dependent F_CFL, F_UPDATE and the debug outputs), so that each member runs the
 // same arithmetic in the batch as alone.
-int member_flags(const p2de_param& p, bool axis_aligned, int precision) {
+int member_flags(const p2de_param& p, bool axis_aligned, bool own_boundaries, int precision) {
   int f = 0;
   switch (p.rhs_type) {
     case P2DE_RHS_LOW_ORDER_POSITIVITY: f |= F_DO_LOW | F_RHSU_FROM_L; break;
@@ -163,6 +163,7 @@ int member_flags(const p2de_param& p, bool axis_aligned, int precision) {
   if (precision == P2DE_PRECISION_MIXED_ACC64) f |= F_ACC64;
   if (p.shock_capture == 1 && (f & (F_DO_LIMIT | F_ZHANG_SHU))) f |= F_SHOCK;
   if (p.low_order_surface_flux == P2DE_FLUX_LAX_FRIEDRICHS_ON_PROJECTED_VAL) f |= F_LFPROJ;
+  if (flux_form(f, p.N, p.ZEROTOL, own_boundaries, precision == P2DE_PRECISION_MIXED)) f |= F_FLUX;
   return f;
 }
 
@@ -175,10 +176,10 @@ struct Slot {
   Layout lay{};
 };
 
-// Task segments of a batch: the members' tasks for the plain and the EXT instantiation of
-// kernel A, then the same members' tasks again for the low-only pass of the TVD bounds.
-// Kernel B runs over segments 0 and 1, which are contiguous.
-enum : int { SEG_PLAIN = 0, SEG_EXT = 1, SEG_LOW_PLAIN = 2, SEG_LOW_EXT = 3, NSEG = 4 };
+// Task segments of a batch: the members' tasks by kind of kernel A (BATCH_*), then the same
+// members' tasks again for the low-only pass of the TVD bounds. Kernel B runs over segments
+// 0-1, its flux form over 2-3, each contiguous; their task counts follow the segments'.
+enum : int { NSEG = 2 * BATCH_KINDS, NT_B = NSEG, NT_FLUX_B = NSEG + 1, NCOUNTS = NSEG + 2 };
 
 double now_s() {
   using namespace std::chrono;
@@ -212,12 +213,12 @@ struct p2de_batch {
   std::vector<uint64_t> table_zerotol;
   int task_cap = 0;
   int sms = 0;
-  int grid_a = 0, grid_x = 0, grid_b = 0;
-  // launch shared memory of the captured graph: plain and EXT kernel A, kernel B
-  size_t smem_a = 0, smem_x = 0, smem_b = 0;
+  int grid_a[BATCH_KINDS] = {}, grid_b = 0, grid_fb = 0;
+  // launch shared memory of the captured graph: kernel A by kind, kernel B
+  size_t smem_a[BATCH_KINDS] = {}, smem_b = 0;
   int seg_off[NSEG] = {}, seg_cnt[NSEG] = {};  // task segments (offsets into d_tasks)
   bool phi_min = false;                         // some member needs the initial min of phi
-  int epb[kMaxN1D + 1] = {};     // elements per block per N1D
+  int epb[kMaxN1D + 1] = {};     // elements per block per N1D (0: each kind's default)
   int layout[kMaxN1D + 1] = {};  // thread layout (p2de_layout) per N1D
   cudaGraphExec_t graph = nullptr;
   bool tasks_dirty = true;
@@ -327,27 +328,33 @@ int validate_solve(const p2de_param* p, const p2de_mesh* m, std::string& why) {
   return P2DE_OK;
 }
 
+// elements per block of a degree's members of a kind
+int kind_epb(const p2de_batch* b, int n1d, int kind) {
+  return b->epb[n1d] > 0 ? b->epb[n1d] : batch_elems_per_block(n1d, kind >= BATCH_FLUX);
+}
+
 // The tasks of one member: elements in runs of the degree's elements per block.
 void member_tasks(const p2de_batch* b, int s, std::vector<BatchTask>& t) {
   const Slot& sl = b->slots[s];
-  const int E = b->epb[sl.n1d];
+  const int E = kind_epb(b, sl.n1d, batch_kind(sl.flags));
   for (int k0 = 0; k0 < sl.prm.K; k0 += E) t.push_back(BatchTask{s, k0, sl.n1d, E, b->layout[sl.n1d]});
 }
 
 // The task list in its segments, largest tasks first within each (work per task grows
-// with elements * N1D^3), and the kernels' shared memory for each instantiation.
-std::vector<BatchTask> build_tasks(p2de_batch* b, size_t* smem_a, size_t* smem_x, size_t* smem_b) {
+// with elements * N1D^3), and the kernels' shared memory for each kind.
+std::vector<BatchTask> build_tasks(p2de_batch* b, size_t smem_a[BATCH_KINDS], size_t* smem_b) {
   std::vector<BatchTask> seg[NSEG];
-  *smem_a = *smem_x = *smem_b = 0;
+  for (int g = 0; g < BATCH_KINDS; ++g) smem_a[g] = 0;
+  *smem_b = 0;
   for (int s = 0; s < b->max_solves; ++s) {
     const Slot& sl = b->slots[s];
     if (!sl.active) continue;
-    const bool ext = sl.flags & kExtFlags, tvd = sl.flags & F_TVD;
-    const int E = b->epb[sl.n1d];
-    (ext ? *smem_x : *smem_a) = std::max(ext ? *smem_x : *smem_a, batch_smem_a(sl.n1d, E, ext));
-    *smem_b = std::max(*smem_b, batch_smem_b(sl.n1d, E));
-    member_tasks(b, s, seg[ext ? SEG_EXT : SEG_PLAIN]);
-    if (tvd) member_tasks(b, s, seg[ext ? SEG_LOW_EXT : SEG_LOW_PLAIN]);
+    const int kind = batch_kind(sl.flags);
+    const int E = kind_epb(b, sl.n1d, kind);
+    smem_a[kind] = std::max(smem_a[kind], batch_smem_a(sl.n1d, E, kind));
+    if (kind < BATCH_FLUX) *smem_b = std::max(*smem_b, batch_smem_b(sl.n1d, E));
+    member_tasks(b, s, seg[kind]);
+    if (sl.flags & F_TVD) member_tasks(b, s, seg[BATCH_KINDS + kind]);
   }
   std::vector<BatchTask> t;
   for (int g = 0; g < NSEG; ++g) {
@@ -359,26 +366,25 @@ std::vector<BatchTask> build_tasks(p2de_batch* b, size_t* smem_a, size_t* smem_x
     b->seg_cnt[g] = (int)seg[g].size();
     t.insert(t.end(), seg[g].begin(), seg[g].end());
   }
-  if (*smem_a == 0) *smem_a = batch_smem_a(2, 1, false);
-  if (*smem_x == 0) *smem_x = batch_smem_a(2, 1, true);
+  for (int g = 0; g < BATCH_KINDS; ++g)
+    if (smem_a[g] == 0) smem_a[g] = batch_smem_a(2, 1, g);
   if (*smem_b == 0) *smem_b = batch_smem_b(2, 1);
   return t;
 }
 
 int upload_tasks(p2de_batch* b) {
-  size_t sa = 0, sx = 0, sb = 0;
+  size_t sa[BATCH_KINDS], sb = 0;
   int cnt_before[NSEG];
   std::memcpy(cnt_before, b->seg_cnt, sizeof cnt_before);
   const bool phi_before = b->phi_min;
-  std::vector<BatchTask> t = build_tasks(b, &sa, &sx, &sb);
+  std::vector<BatchTask> t = build_tasks(b, sa, &sb);
   b->phi_min = false;
   for (int s = 0; s < b->max_solves; ++s)
     if (b->slots[s].active && (b->slots[s].flags & F_MIN_ENTROPY) && (b->slots[s].flags & F_RELAXED)) b->phi_min = true;
-  bool relaunch = sa != b->smem_a || sx != b->smem_x || sb != b->smem_b || b->phi_min != phi_before;
+  bool relaunch = std::memcmp(sa, b->smem_a, sizeof sa) != 0 || sb != b->smem_b || b->phi_min != phi_before;
   for (int g = 0; g < NSEG; ++g) relaunch |= (cnt_before[g] > 0) != (b->seg_cnt[g] > 0);
   if (relaunch) {  // launch configuration or the set of launches changes: new capture
-    b->smem_a = sa;
-    b->smem_x = sx;
+    std::memcpy(b->smem_a, sa, sizeof sa);
     b->smem_b = sb;
     if (b->graph) {
       BCK(cudaStreamSynchronize(b->stream));
@@ -402,15 +408,21 @@ int upload_tasks(p2de_batch* b) {
   }
   int nt = (int)t.size();
   if (nt) BCK(cudaMemcpyAsync(b->d_tasks, t.data(), sizeof(BatchTask) * nt, cudaMemcpyHostToDevice, b->stream));
-  // task counts: segments 0..3, then segments 0 and 1 together (kernel B)
-  int counts[NSEG + 1];
+  int counts[NCOUNTS];
   for (int g = 0; g < NSEG; ++g) counts[g] = b->seg_cnt[g];
-  counts[NSEG] = b->seg_cnt[SEG_PLAIN] + b->seg_cnt[SEG_EXT];
+  counts[NT_B] = b->seg_cnt[BATCH_PLAIN] + b->seg_cnt[BATCH_EXT];
+  counts[NT_FLUX_B] = b->seg_cnt[BATCH_FLUX] + b->seg_cnt[BATCH_FLUX_EXT];
   BCK(cudaMemcpyAsync(b->d_ntasks, counts, sizeof counts, cudaMemcpyHostToDevice, b->stream));
   BCK(cudaMemcpyAsync(b->d_active, b->active.data(), b->max_solves, cudaMemcpyHostToDevice, b->stream));
   BCK(cudaStreamSynchronize(b->stream));  // the host vectors above are temporaries
   b->tasks_dirty = false;
   return P2DE_OK;
+}
+
+// whether kernel B (or its flux form) has tasks
+bool has_b(const p2de_batch* b, bool flux) {
+  const int g = flux ? BATCH_FLUX : BATCH_PLAIN;
+  return b->seg_cnt[g] + b->seg_cnt[g + 1] > 0;
 }
 
 // One step: the step begin, then per stage, in the one-solve path's order, the initial
@@ -422,20 +434,18 @@ int enqueue_batch_step(p2de_batch* b) {
   for (int stage = 1; stage <= 3; ++stage) {
     unsigned* ctr = b->d_counters + kBatchCountersPerStage * (stage - 1);
     if (stage == 1 && b->phi_min) BCK(launch_batch_phi_min(b->d_solves, b->d_active, b->max_solves, b->stream));
-    struct Pass {
-      int seg, mode;
-      bool ext;
-    } passes[4] = {{SEG_LOW_PLAIN, BATCH_A_LOW_ONLY, false},
-                   {SEG_LOW_EXT, BATCH_A_LOW_ONLY, true},
-                   {SEG_PLAIN, BATCH_A_FULL, false},
-                   {SEG_EXT, BATCH_A_FULL, true}};
-    for (int i = 0; i < 4; ++i) {
-      const Pass& q = passes[i];
-      if (b->seg_cnt[q.seg] == 0) continue;
-      BCK(launch_batch_a(b->mixed, q.ext, q.mode, q.ext ? b->grid_x : b->grid_a, q.ext ? b->smem_x : b->smem_a,
-                         b->d_solves, b->d_tasks + b->seg_off[q.seg], b->d_ntasks + q.seg, ctr + i, stage, b->stream));
+    for (int i = 0; i < NSEG; ++i) {  // the low-only passes, then the full ones
+      const int kind = i % BATCH_KINDS, low = i < BATCH_KINDS, g = low ? BATCH_KINDS + kind : kind;
+      if (b->seg_cnt[g] == 0) continue;
+      BCK(launch_batch_a(b->mixed, kind, low ? BATCH_A_LOW_ONLY : BATCH_A_FULL, b->grid_a[kind], b->smem_a[kind],
+                         b->d_solves, b->d_tasks + b->seg_off[g], b->d_ntasks + g, ctr + i, stage, b->stream));
     }
-    BCK(launch_batch_b(b->grid_b, b->smem_b, b->d_solves, b->d_tasks, b->d_ntasks + NSEG, ctr + 4, stage, b->stream));
+    if (has_b(b, false))
+      BCK(launch_batch_b(false, b->grid_b, b->smem_b, b->d_solves, b->d_tasks, b->d_ntasks + NT_B, ctr + NSEG, stage,
+                         b->stream));
+    if (has_b(b, true))
+      BCK(launch_batch_b(true, b->grid_fb, 0, b->d_solves, b->d_tasks + b->seg_off[BATCH_FLUX],
+                         b->d_ntasks + NT_FLUX_B, ctr + NSEG + 1, stage, b->stream));
   }
   return P2DE_OK;
 }
@@ -444,18 +454,22 @@ int enqueue_batch_step(p2de_batch* b) {
 int step_launch_count(const p2de_batch* b) {
   int n = 1 + (b->phi_min ? 1 : 0);
   for (int g = 0; g < NSEG; ++g) n += 3 * (b->seg_cnt[g] > 0 ? 1 : 0);
-  return n + 3;
+  return n + 3 * (has_b(b, false) ? 1 : 0) + 3 * (has_b(b, true) ? 1 : 0);
 }
 
 // persistent grids: resident blocks per SM at the current shared memory, times the SMs
 int size_grids(p2de_batch* b) {
-  int bpa = 0, bpb = 0, bpx = 0, bpb2 = 0;
-  BCK(batch_occupancy(b->mixed, false, b->smem_a, b->smem_b, &bpa, &bpb));
-  BCK(batch_occupancy(b->mixed, true, b->smem_x, b->smem_b, &bpx, &bpb2));
-  if (bpa < 1 || bpb < 1 || bpx < 1) return bfail(b, P2DE_ERR_CUDA, "batched kernels do not fit an SM");
-  b->grid_a = b->sms * bpa;
-  b->grid_x = b->sms * bpx;
-  b->grid_b = b->sms * bpb;
+  int bp = 0;
+  for (int g = 0; g < BATCH_KINDS; ++g) {
+    BCK(batch_occupancy_a(b->mixed, g, b->smem_a[g], &bp));
+    if (bp < 1) return bfail(b, P2DE_ERR_CUDA, "batched kernels do not fit an SM");
+    b->grid_a[g] = b->sms * bp;
+  }
+  for (bool flux : {false, true}) {
+    BCK(batch_occupancy_b(flux, b->smem_b, &bp));
+    if (bp < 1) return bfail(b, P2DE_ERR_CUDA, "batched kernels do not fit an SM");
+    (flux ? b->grid_fb : b->grid_b) = b->sms * bp;
+  }
   return P2DE_OK;
 }
 
@@ -509,7 +523,7 @@ int p2de_batch_create(int device, int32_t precision, size_t pool_bytes, int32_t 
     return bail(P2DE_ERR_CUDA);
   if (b->pool.init(pool_bytes) != cudaSuccess) return bail(P2DE_ERR_OUT_OF_MEMORY);
   if (balloc(b, &b->d_solves, max_solves) != cudaSuccess || balloc(b, &b->d_active, max_solves) != cudaSuccess ||
-      balloc(b, &b->d_ntasks, NSEG + 1) != cudaSuccess || balloc(b, &b->d_counters, kBatchCounters + 1) != cudaSuccess ||
+      balloc(b, &b->d_ntasks, NCOUNTS) != cudaSuccess || balloc(b, &b->d_counters, kBatchCounters + 1) != cudaSuccess ||
       balloc(b, &b->d_scal, (size_t)max_solves * S_NSCAL) != cudaSuccess ||
       balloc(b, &b->d_dtmin, max_solves) != cudaSuccess || balloc(b, &b->d_minrec, (size_t)6 * max_solves) != cudaSuccess ||
       balloc(b, &b->d_status, max_solves) != cudaSuccess || balloc(b, &b->d_work, 8) != cudaSuccess ||
@@ -532,7 +546,6 @@ int p2de_batch_create(int device, int32_t precision, size_t pool_bytes, int32_t 
   cudaDeviceProp prop;
   if (cudaGetDeviceProperties(&prop, device) != cudaSuccess) return bail(P2DE_ERR_CUDA);
   b->sms = prop.multiProcessorCount;
-  for (int n = 2; n <= kMaxN1D; ++n) b->epb[n] = batch_elems_per_block(n);
   b->task_cap = 0;
   if (cudaStreamSynchronize(b->stream) != cudaSuccess) return bail(P2DE_ERR_CUDA);
   *out = b;
@@ -606,7 +619,9 @@ int p2de_batch_add(p2de_batch* b, const p2de_param* p, const p2de_mesh* m, const
   StageArgs a{};
   a.K = p->K;
   a.nstage = 1;
-  const int f = member_flags(*p, aa, b->precision);
+  const bool own = own_faces(m->mapI, m->nI, m->mapP) && own_faces(m->mapO, m->nO, m->mapP) &&
+                   own_faces(m->mapW, m->nW, m->mapP) && own_faces(m->mapS, m->nS, m->mapP);
+  const int f = member_flags(*p, aa, own, b->precision);
   a.flags = f;
   set_shock_capture(a, p->N, p->shock_capture_a, p->shock_capture_c);
   set_bound_constants(a, p->N, p->t0, p->POSTOL, p->bound_beta);
@@ -634,8 +649,7 @@ int p2de_batch_add(p2de_batch* b, const p2de_param* p, const p2de_mesh* m, const
     a.shock_post[c] = m->shock_post[c];
     a.shock_pre[c] = m->shock_pre[c];
   }
-  a.gamma = p->gamma;
-  a.gm1 = p->gamma - 1.0;
+  set_gas(a, p->gamma);
   a.CFL = p->CFL;
   a.dt0 = p->dt0;
   a.T = p->T;
@@ -732,7 +746,7 @@ int p2de_batch_get_layout(p2de_batch* b, int32_t N, int32_t* layout) {
 
 int p2de_batch_get_elements_per_block(p2de_batch* b, int32_t N, int32_t* epb, int32_t* epb_max) {
   if (!b || N < 1 || N + 1 > kMaxN1D) return P2DE_ERR_INVALID_ARGUMENT;
-  if (epb) *epb = b->epb[N + 1];
+  if (epb) *epb = kind_epb(b, N + 1, BATCH_FLUX);
   if (epb_max) *epb_max = batch_elems_per_block_max(N + 1);
   return P2DE_OK;
 }
@@ -785,42 +799,42 @@ int p2de_batch_autotune(p2de_batch* b, int32_t best_epb[5]) {
     bool present = false;
     for (int s = 0; s < b->max_solves; ++s) present |= b->slots[s].active && b->slots[s].n1d == n1d;
     if (!present) continue;
-    const int emax = batch_elems_per_block_max(n1d), edef = batch_elems_per_block(n1d);
-    int best = b->epb[n1d], best_layout = b->layout[n1d];
+    const int emax = batch_elems_per_block_max(n1d), edef = batch_elems_per_block(n1d, true);
+    int best = edef, best_layout = b->layout[n1d];
     double bms = 1e30;
     for (int lay : {(int)P2DE_LAYOUT_FLAT, (int)P2DE_LAYOUT_LINES_PER_WARP})
     for (int e : {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, edef}) {
       if (e > emax) continue;
-      // this degree's members, plain and EXT instantiation, full pass at stage 2
-      std::vector<BatchTask> t[2];
+      // this degree's members by kind, full pass at stage 2
+      std::vector<BatchTask> t[BATCH_KINDS], all;
       for (int s = 0; s < b->max_solves; ++s) {
         const Slot& sl = b->slots[s];
         if (!sl.active || sl.n1d != n1d) continue;
-        const int x = (sl.flags & kExtFlags) ? 1 : 0;
-        for (int k0 = 0; k0 < sl.prm.K; k0 += e) t[x].push_back(BatchTask{s, k0, n1d, e, lay});
+        for (int k0 = 0; k0 < sl.prm.K; k0 += e) t[batch_kind(sl.flags)].push_back(BatchTask{s, k0, n1d, e, lay});
       }
-      int grid[2] = {0, 0}, nt[2] = {(int)t[0].size(), (int)t[1].size()};
-      size_t sm[2] = {batch_smem_a(n1d, e, false), batch_smem_a(n1d, e, true)};
+      int grid[BATCH_KINDS] = {}, nt[BATCH_KINDS], off[BATCH_KINDS];
+      size_t sm[BATCH_KINDS];
       bool fits = true;
-      for (int x = 0; x < 2; ++x) {
+      for (int x = 0; x < BATCH_KINDS; ++x) {
+        nt[x] = (int)t[x].size();
+        off[x] = (int)all.size();
+        sm[x] = batch_smem_a(n1d, e, x);
+        all.insert(all.end(), t[x].begin(), t[x].end());
         if (!nt[x]) continue;
-        int bpa = 0, bpb = 0;
-        cudaError_t ce = batch_occupancy(b->mixed, x == 1, sm[x], batch_smem_b(n1d, e), &bpa, &bpb);
-        if (ce != cudaSuccess || bpa < 1) fits = false;
+        int bpa = 0;
+        if (batch_occupancy_a(b->mixed, x, sm[x], &bpa) != cudaSuccess || bpa < 1) fits = false;
         grid[x] = std::min(b->sms * bpa, nt[x]);
       }
       if (!fits) continue;
-      std::vector<BatchTask> all = t[0];
-      all.insert(all.end(), t[1].begin(), t[1].end());
       BCK(cudaMemcpyAsync(b->d_tasks, all.data(), sizeof(BatchTask) * all.size(), cudaMemcpyHostToDevice, b->stream));
       BCK(cudaMemcpyAsync(b->d_ntasks, nt, sizeof nt, cudaMemcpyHostToDevice, b->stream));
       float tot = 0.f;
       for (int rep = 0; rep < 4; ++rep) {
         BCK(cudaEventRecord(e0, b->stream));
-        for (int x = 0; x < 2; ++x) {
+        for (int x = 0; x < BATCH_KINDS; ++x) {
           if (!nt[x]) continue;
           BCK(cudaMemsetAsync(counter, 0, sizeof(unsigned), b->stream));
-          BCK(launch_batch_a(b->mixed, x == 1, BATCH_A_FULL, grid[x], sm[x], b->d_solves, b->d_tasks + (x ? nt[0] : 0),
+          BCK(launch_batch_a(b->mixed, x, BATCH_A_FULL, grid[x], sm[x], b->d_solves, b->d_tasks + off[x],
                              b->d_ntasks + x, counter, 2, b->stream));
           b->launches += 1;
         }

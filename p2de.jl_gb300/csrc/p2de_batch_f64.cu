@@ -1,33 +1,47 @@
-// Batched stage kernels, FP64 flux differencing; kernel B and the step begin.
+// Batched stage kernels, FP64 flux differencing; kernels B and the step begin.
 #define P2DE_BATCH_COMMON_KERNELS
 #include "p2de_batch_kernels.cuh"
-#include "p2de_batch_launch.h"
 
 namespace p2de {
 
 cudaError_t batch_prepare_f64() {
-  cudaError_t e = cudaFuncSetAttribute(k_batch_a<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)kBatchSmemAMax);
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(k_batch_a<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBatchSmemXMax);
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(k_batch_b, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBatchSmemBMax);
+  const struct {
+    const void* f;
+    size_t smem;
+  } k[] = {{(const void*)k_batch_a<double, false>, kBatchSmemAMax},
+           {(const void*)k_batch_a<double, true>, kBatchSmemXMax},
+           {(const void*)k_batch_flux_a<double, false>, kBatchSmemFluxMax<false>},
+           {(const void*)k_batch_flux_a<double, true>, kBatchSmemFluxMax<true>},
+           {(const void*)k_batch_b, kBatchSmemBMax}};
+  for (const auto& q : k) {
+    cudaError_t e = cudaFuncSetAttribute(q.f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)q.smem);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
-cudaError_t batch_occupancy_f64(bool ext, size_t smem_a, size_t smem_b, int* bpa, int* bpb) {
-  cudaError_t e = ext ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(bpa, k_batch_a<double, true>, kBatchThreads, smem_a)
-                      : cudaOccupancyMaxActiveBlocksPerMultiprocessor(bpa, k_batch_a<double, false>, kBatchThreads, smem_a);
-  if (e != cudaSuccess) return e;
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bpb, k_batch_b, kBatchThreads, smem_b);
+cudaError_t batch_occupancy_a_f64(int kind, size_t smem, int* bpa) {
+  const void* k[] = {(const void*)k_batch_a<double, false>, (const void*)k_batch_a<double, true>,
+                     (const void*)k_batch_flux_a<double, false>, (const void*)k_batch_flux_a<double, true>};
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bpa, k[kind], kBatchThreads, smem);
 }
 
-cudaError_t launch_batch_a_f64(bool ext, int mode, int grid, size_t smem, const StageArgs* solves,
+cudaError_t batch_occupancy_b(bool flux, size_t smem, int* bpb) {
+  return flux ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(bpb, k_batch_flux_b, kBatchThreads, 0)
+              : cudaOccupancyMaxActiveBlocksPerMultiprocessor(bpb, k_batch_b, kBatchThreads, smem);
+}
+
+cudaError_t launch_batch_a_f64(int kind, int mode, int grid, size_t smem, const StageArgs* solves,
                                const BatchTask* tasks, const int* ntasks, unsigned* counter, int nstage,
                                cudaStream_t st) {
-  if (ext)
+  if (kind == BATCH_EXT)
     k_batch_a<double, true><<<grid, kBatchThreads, smem, st>>>(solves, tasks, ntasks, counter, nstage, mode);
-  else
+  else if (kind == BATCH_PLAIN)
     k_batch_a<double, false><<<grid, kBatchThreads, smem, st>>>(solves, tasks, ntasks, counter, nstage, mode);
+  else if (kind == BATCH_FLUX_EXT)
+    k_batch_flux_a<double, true><<<grid, kBatchThreads, smem, st>>>(solves, tasks, ntasks, counter, nstage, mode);
+  else
+    k_batch_flux_a<double, false><<<grid, kBatchThreads, smem, st>>>(solves, tasks, ntasks, counter, nstage, mode);
   return cudaGetLastError();
 }
 
@@ -36,9 +50,12 @@ cudaError_t launch_batch_phi_min(const StageArgs* solves, const uint8_t* active,
   return cudaGetLastError();
 }
 
-cudaError_t launch_batch_b(int grid, size_t smem, const StageArgs* solves, const BatchTask* tasks, const int* ntasks,
-                           unsigned* counter, int nstage, cudaStream_t st) {
-  k_batch_b<<<grid, kBatchThreads, smem, st>>>(solves, tasks, ntasks, counter, nstage);
+cudaError_t launch_batch_b(bool flux, int grid, size_t smem, const StageArgs* solves, const BatchTask* tasks,
+                           const int* ntasks, unsigned* counter, int nstage, cudaStream_t st) {
+  if (flux)
+    k_batch_flux_b<<<grid, kBatchThreads, 0, st>>>(solves, tasks, ntasks, counter, nstage);
+  else
+    k_batch_b<<<grid, kBatchThreads, smem, st>>>(solves, tasks, ntasks, counter, nstage);
   return cudaGetLastError();
 }
 
@@ -49,35 +66,45 @@ cudaError_t launch_batch_begin(const StageArgs* solves, const uint8_t* active, i
   return cudaGetLastError();
 }
 
-int batch_elems_per_block(int n1d) {
+template <int N1D>
+static size_t smem_a_of(int epb, int kind) {
+  switch (kind) {
+    case BATCH_PLAIN: return Cfg<N1D>::smem_a(epb);
+    case BATCH_EXT: return Cfg<N1D>::smem_x(epb);
+    case BATCH_FLUX: return FluxCfg<N1D>::template smem<false>(epb);
+    default: return FluxCfg<N1D>::template smem<true>(epb);
+  }
+}
+
+int batch_elems_per_block(int n1d, bool flux) {
   switch (n1d) {
-    case 2: return Cfg<2>::E;
-    case 3: return Cfg<3>::E;
-    case 4: return Cfg<4>::E;
-    case 5: return Cfg<5>::E;
-    case 6: return Cfg<6>::E;
+    case 2: return flux ? FluxCfg<2>::E : Cfg<2>::E;
+    case 3: return flux ? FluxCfg<3>::E : Cfg<3>::E;
+    case 4: return flux ? FluxCfg<4>::E : Cfg<4>::E;
+    case 5: return flux ? FluxCfg<5>::E : Cfg<5>::E;
+    case 6: return flux ? FluxCfg<6>::E : Cfg<6>::E;
   }
   return 0;
 }
 
 int batch_elems_per_block_max(int n1d) {
   switch (n1d) {
-    case 2: return Cfg<2>::E_MAX;
-    case 3: return Cfg<3>::E_MAX;
-    case 4: return Cfg<4>::E_MAX;
-    case 5: return Cfg<5>::E_MAX;
-    case 6: return Cfg<6>::E_MAX;
+    case 2: return cmin(Cfg<2>::E_MAX, FluxCfg<2>::E_MAX);
+    case 3: return cmin(Cfg<3>::E_MAX, FluxCfg<3>::E_MAX);
+    case 4: return cmin(Cfg<4>::E_MAX, FluxCfg<4>::E_MAX);
+    case 5: return cmin(Cfg<5>::E_MAX, FluxCfg<5>::E_MAX);
+    case 6: return cmin(Cfg<6>::E_MAX, FluxCfg<6>::E_MAX);
   }
   return 0;
 }
 
-size_t batch_smem_a(int n1d, int epb, bool ext) {
+size_t batch_smem_a(int n1d, int epb, int kind) {
   switch (n1d) {
-    case 2: return ext ? Cfg<2>::smem_x(epb) : Cfg<2>::smem_a(epb);
-    case 3: return ext ? Cfg<3>::smem_x(epb) : Cfg<3>::smem_a(epb);
-    case 4: return ext ? Cfg<4>::smem_x(epb) : Cfg<4>::smem_a(epb);
-    case 5: return ext ? Cfg<5>::smem_x(epb) : Cfg<5>::smem_a(epb);
-    case 6: return ext ? Cfg<6>::smem_x(epb) : Cfg<6>::smem_a(epb);
+    case 2: return smem_a_of<2>(epb, kind);
+    case 3: return smem_a_of<3>(epb, kind);
+    case 4: return smem_a_of<4>(epb, kind);
+    case 5: return smem_a_of<5>(epb, kind);
+    case 6: return smem_a_of<6>(epb, kind);
   }
   return 0;
 }

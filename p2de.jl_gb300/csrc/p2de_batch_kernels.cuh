@@ -10,6 +10,8 @@
 #include <stdint.h>
 
 #include "p2de_args.h"
+#include "p2de_batch_launch.h"
+#include "p2de_flux.cuh"
 #include "p2de_stage.cuh"
 
 namespace p2de {
@@ -35,6 +37,11 @@ constexpr size_t kBatchSmemXMax =
     smax(smax(smax(Cfg<2>::smem_x(Cfg<2>::E_MAX), Cfg<3>::smem_x(Cfg<3>::E_MAX)),
               smax(Cfg<4>::smem_x(Cfg<4>::E_MAX), Cfg<5>::smem_x(Cfg<5>::E_MAX))),
          Cfg<6>::smem_x(Cfg<6>::E_MAX));
+template <bool EXT>
+constexpr size_t kBatchSmemFluxMax =
+    smax(smax(smax(FluxCfg<2>::smem<EXT>(FluxCfg<2>::E_MAX), FluxCfg<3>::smem<EXT>(FluxCfg<3>::E_MAX)),
+              smax(FluxCfg<4>::smem<EXT>(FluxCfg<4>::E_MAX), FluxCfg<5>::smem<EXT>(FluxCfg<5>::E_MAX))),
+         FluxCfg<6>::smem<EXT>(FluxCfg<6>::E_MAX));
 constexpr size_t kBatchSmemBMax =
     smax(smax(smax(Cfg<2>::smem_b(Cfg<2>::E_MAX), Cfg<3>::smem_b(Cfg<3>::E_MAX)),
               smax(Cfg<4>::smem_b(Cfg<4>::E_MAX), Cfg<5>::smem_b(Cfg<5>::E_MAX))),
@@ -44,8 +51,9 @@ constexpr size_t kBatchSmemBMax =
 // after the low-order RHS and stores the low-order densities (the one-solve path's first
 // kernel A launch of such a stage)
 enum : int { BATCH_A_FULL = 0, BATCH_A_LOW_ONLY = 1 };
-// task counters per step: kBatchCountersPerStage per stage (kernel A passes and kernel B)
-constexpr int kBatchCountersPerStage = 5;
+// task counters per step: per stage the two kernel A passes of each kind (BATCH_*) and the
+// two kernels B
+constexpr int kBatchCountersPerStage = 2 * BATCH_KINDS + 2;
 constexpr int kBatchCounters = 3 * kBatchCountersPerStage;
 
 // Fetches the next task; returns false when the list is exhausted. The solve's
@@ -98,6 +106,26 @@ __global__ void __launch_bounds__(kBatchThreads) k_batch_a(const StageArgs* solv
   }
 }
 
+// the members whose stage kernels run in flux form (p2de_flux.cuh)
+template <typename TH, bool EXT>
+__global__ void __launch_bounds__(kBatchThreads) k_batch_flux_a(const StageArgs* solves, const BatchTask* tasks,
+                                                                const int* ntasks, unsigned* counter, int nstage,
+                                                                int mode) {
+  extern __shared__ __align__(16) double sm[];
+  __shared__ StageArgs sa;
+  __shared__ int s_task;
+  BatchTask tk;
+  while (batch_next(solves, tasks, ntasks, counter, nstage, sa, tk, s_task, mode)) {
+    switch (tk.n1d) {
+      case 2: flux_a_body<2, TH, EXT>(sa, tk.k0, sm); break;
+      case 3: flux_a_body<3, TH, EXT>(sa, tk.k0, sm); break;
+      case 4: flux_a_body<4, TH, EXT>(sa, tk.k0, sm); break;
+      case 5: flux_a_body<5, TH, EXT>(sa, tk.k0, sm); break;
+      case 6: flux_a_body<6, TH, EXT>(sa, tk.k0, sm); break;
+    }
+  }
+}
+
 // Kernel B and the step begin are defined in one translation unit only.
 #ifdef P2DE_BATCH_COMMON_KERNELS
 __global__ void __launch_bounds__(kBatchThreads) k_batch_b(const StageArgs* solves, const BatchTask* tasks,
@@ -117,7 +145,23 @@ __global__ void __launch_bounds__(kBatchThreads) k_batch_b(const StageArgs* solv
   }
 }
 
-// Step begin for every slot (SSPRK33.jl:126 per solve) and reset of the six task
+__global__ void __launch_bounds__(kBatchThreads) k_batch_flux_b(const StageArgs* solves, const BatchTask* tasks,
+                                                                const int* ntasks, unsigned* counter, int nstage) {
+  __shared__ StageArgs sa;
+  __shared__ int s_task;
+  BatchTask tk;
+  while (batch_next(solves, tasks, ntasks, counter, nstage, sa, tk, s_task)) {
+    switch (tk.n1d) {
+      case 2: flux_b_body<2>(sa, tk.k0); break;
+      case 3: flux_b_body<3>(sa, tk.k0); break;
+      case 4: flux_b_body<4>(sa, tk.k0); break;
+      case 5: flux_b_body<5>(sa, tk.k0); break;
+      case 6: flux_b_body<6>(sa, tk.k0); break;
+    }
+  }
+}
+
+// Step begin for every slot (SSPRK33.jl:126 per solve) and reset of the task
 // counters of the step. scal/dtmin/minrec/status are slot-indexed arrays.
 __global__ void k_batch_begin(const StageArgs* solves, const uint8_t* active, int nslots, unsigned* counters) {
   int s = blockIdx.x * blockDim.x + threadIdx.x;

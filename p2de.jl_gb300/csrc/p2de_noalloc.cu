@@ -215,8 +215,7 @@ extern "C" int p2de_rhs_noalloc(const p2de_param* prm, const p2de_device_mesh* m
     a.shock_post[c] = mesh->shock_post[c];
     a.shock_pre[c] = mesh->shock_pre[c];
   }
-  a.gamma = prm->gamma;
-  a.gm1 = prm->gamma - 1.0;
+  set_gas(a, prm->gamma);
   a.CFL = prm->CFL;
   a.dt0 = prm->dt0;
   a.T = prm->T;

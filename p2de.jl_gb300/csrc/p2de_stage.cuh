@@ -146,11 +146,15 @@ __device__ __forceinline__ double rcp(double x) {
 // result). 15 FP64 instructions against 31 for log(); within one unit in the last place of
 // the correctly rounded value (checked against an extended-precision log on 4M arguments
 // from 1e-9 to 2e8 and around 1), like log(). Positive normal finite x; anything else
-// goes to log().
+// goes to log(). HALF: log(x/2), the same bits as log_fast(0.5 x) (the halving is in the
+// exponent).
+template <bool HALF = false>
 __device__ __forceinline__ double log_fast(double x, const OpTable& op) {
   const long long b = __double_as_longlong(x);
-  if ((unsigned long long)(b - 0x0010000000000000LL) >= 0x7fe0000000000000ULL) return log(x);
-  long long k = (b >> 52) - 1023;
+  if ((unsigned long long)(b - (HALF ? 0x0020000000000000LL : 0x0010000000000000LL)) >=
+      (HALF ? 0x7fd0000000000000ULL : 0x7fe0000000000000ULL))
+    return log(HALF ? 0.5 * x : x);
+  long long k = (b >> 52) - (HALF ? 1024 : 1023);
   long long mb = (b & 0x000fffffffffffffLL) | 0x3ff0000000000000LL;  // m in [1, 2)
   if (((mb >> 44) & 0xff) >= 106) {  // m >= 1 + 106/256: use m/2 in [0.707, 1)
     mb -= 0x0010000000000000LL;

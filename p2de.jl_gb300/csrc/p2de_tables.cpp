@@ -361,6 +361,12 @@ int build_op_table(int N, double zerotol, OpTable* T, int basis) {
       T->lga_count[ax][m] = (int8_t)(c + 1);
     }
   }
+  for (int i = 0; i < n; ++i) T->rw1D[i] = 1.0 / w[i];
+  const int ppl = n * (n - 1) / 2;  // pairs per line; the tangential node of pair q is (q / ppl) % n
+  for (int q = 0; q < T->nph; ++q) {
+    T->hpc[q] = -T->hp_S[q] / w[(q / ppl) % n];
+    T->hpcf[q] = (float)T->hpc[q];
+  }
   return 0;
 }
 

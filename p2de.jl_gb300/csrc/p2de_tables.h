@@ -68,6 +68,11 @@ struct OpTable {
   // the same two parts (42 significant bits, so that k log2_hi is exact for |k| < 2048)
   double logtab[kLogTabN][3];
   double ln2_hi, ln2_lo;
+  // flux form (p2de_flux.cuh): 1/w1D, and per high-order pair -hp_S / w of its line's
+  // tangential weight w (FP64, FP32)
+  double rw1D[kMaxN1D];
+  double hpc[kMaxPairsHi];
+  float hpcf[kMaxPairsHi];
 };
 
 // Builds the table for polynomial degree N (1..5) on the LGL (basis 0) or Gauss (basis 1)
