@@ -37,6 +37,15 @@ __device__ __forceinline__ double dsub(double a, double b) { return __dsub_rn(a,
 __device__ __forceinline__ double dmul(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double dfma(double a, double b, double c) { return __fma_rn(a, b, c); }
 
+// x/2 and 2x on the integer pipe: a step of the exponent where x and the result are normal
+__device__ __forceinline__ double scale_exponent(double x, int step) {
+  const int hi = __double2hiint(x), ef = hi & 0x7ff00000;
+  if ((unsigned)(ef - 0x00200000) < 0x7fb00000u) return __hiloint2double(hi + step, __double2loint(x));
+  return is_zero_bits(x) ? x : __dmul_rn(step < 0 ? 0.5 : 2.0, x);
+}
+__device__ __forceinline__ double half(double x) { return scale_exponent(x, -0x00100000); }
+__device__ __forceinline__ double twice(double x) { return scale_exponent(x, 0x00100000); }
+
 // > 0 and not NaN, by the bits
 __device__ __forceinline__ bool positive_bits(double x) {
   const long long b = __double_as_longlong(x);
@@ -95,11 +104,15 @@ struct FluxCfg {
 };
 
 // fS(Dim2) (compressible_Navier_Stokes.jl:220-249) along axis ax for line nodes a and b, in
-// FP64: one reciprocal gives 1/(beta_a + beta_b), and the two quotients of the log means.
+// FP64: one reciprocal gives 1/(beta_a + beta_b) and the two quotients of the log means.
 // The log mean's branch test |da/aavg| < 1e-4 is decided from the exponents of da and of the
 // sum where they settle it (all but two of them), else as written. In its series branch
 // x = da/aavg has x^2 < 1e-8, so the x^4 and x^6 terms of the series (and of its reciprocal,
 // for betalog) are below 2^-53 and are not formed.
+// |x| in [2^-999, 2^1000)
+__device__ __forceinline__ bool mid_exponent(double x) {
+  return (unsigned)((__double2hiint(x) & 0x7ff00000) - (24 << 20)) < (1999u << 20);
+}
 struct PairState {
   double rho, vn, vt, hn, ht, beta, lr, lb;  // velocities normal and tangential to the axis, and halves
 };
@@ -117,10 +130,19 @@ __device__ __forceinline__ void fS_line(double ig, const PairState& a, const Pai
   const bool ser_r = series_branch(dr, sr), ser_b = series_branch(db, sb);
   const double den_r = ser_r ? sr : dsub(a.lr, b.lr);
   const double den_b = ser_b ? sb : db;
-  const double t = dmul(den_r, den_b);
-  const double r = rcp(dmul(t, sb));
-  const double isb = dmul(t, r), q = dmul(sb, r);
-  const double x = dmul(dr, dmul(den_b, q));
+  const double t = dmul(den_r, den_b), D = dmul(t, sb);
+  double isb, idr, idb;  // 1/sb, 1/den_r, 1/den_b
+  if (mid_exponent(t) && mid_exponent(D)) {
+    const double r = rcp(D), q = dmul(sb, r);
+    isb = dmul(t, r);
+    idr = dmul(den_b, q);
+    idb = dmul(den_r, q);
+  } else {  // the products leave the range of doubles
+    isb = rcp(sb);
+    idr = rcp(den_r);
+    idb = rcp(den_b);
+  }
+  const double x = dmul(dr, idr);
   double rl = -x;                  // rho log mean
   double nb = dsub(b.lb, a.lb);    // numerator of 1/beta log mean
   if (ser_r) rl = dmul(sr, dfma(dmul(x, x), -0.4, 0.5));
@@ -128,7 +150,7 @@ __device__ __forceinline__ void fS_line(double ig, const PairState& a, const Pai
     const double y = dmul(db, isb);
     nb = dfma(dmul(y, y), 1.6, 2.0);
   }
-  const double ilb = dmul(nb, dmul(den_r, q));
+  const double ilb = dmul(nb, idb);
   const double pa = dmul(sr, isb);
   const double un = dadd(a.hn, b.hn), ut = dadd(a.ht, b.ht);
   const double w = dfma(a.vt, b.ht, dmul(a.vn, b.hn));
@@ -163,7 +185,7 @@ __device__ __forceinline__ double rhoe_root(const double* U, const double* dF, d
   const double disc = dfma(b, b, -dmul(a4, c));
   double l = 1.0;
   if (disc >= 0.0) {
-    const double sq = __dsqrt_rn(disc);
+    const double sq = sqrt_rn(disc);
     const double k = dmul(r2a, is);
     const double r1 = dmul(dsub(sq, b), k), r2 = dmul(dsub(-b, sq), k);
     if (r1 > ZEROTOL && r2 > ZEROTOL)
@@ -195,7 +217,7 @@ __device__ __forceinline__ void line_node(LineNode& q, double hn, double ht, dou
   q.ft = dmul(q.U[1], ht);
   q.fe = dmul(hn, dfma(2.0, ph, q.U[3]));
   const double pe = dfma(-q.U[1], hn, q.U[3]);
-  q.wh = dadd(fabs(hn), __dsqrt_rn(dmul(pe, crr)));
+  q.wh = dadd(fabs(hn), sqrt_rn(dmul(pe, crr)));
 }
 
 // The body for the elements k0 .. k0 + epb - 1 of the solve `a`; early returns are uniform
@@ -246,7 +268,7 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
     U[2 * Nq] = m2;
     U[3 * Nq] = En;
     double* W = base + C::O_W + m;
-    const double rr = rcp(rho), hr = dmul(0.5, rr);
+    const double rr = rcp(rho), hr = half(rr);
     const double hu = dmul(m1, hr), hv = dmul(m2, hr);
     // p to the bits of the nodal form: log means of nearly equal states amplify its last bit
     const double p = dmul(a.gm1, dfma(-0.5, dmul(dfma(m1, m1, dmul(m2, m2)), rr), En));
@@ -255,7 +277,7 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
     if (!positive_bits(rho) || !positive_bits(p)) atomicOr(a.status, ST_NOT_POSITIVE);
     W[C::W_HU * Nq] = hu;
     W[C::W_HV * Nq] = hv;
-    W[C::W_PH * Nq] = dmul(0.5, p);
+    W[C::W_PH * Nq] = half(p);
     W[C::W_CRR * Nq] = dmul(a.cws, rr);
     if (EXT && (flags & F_RELAXED) || (flags & F_SHOCK)) W[C::W_IND * Nq] = dmul(rho, p);  // shock_capture.jl:92-103
     if (F32) {
@@ -268,8 +290,8 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
       Wf[3 * Nq] = rf / (2.0f * (float)p);
     } else {
       const double beta = dmul(rho, rcp(p));  // 2 beta of the reference
-      W[C::W_U * Nq] = dadd(hu, hu);
-      W[C::W_V * Nq] = dadd(hv, hv);
+      W[C::W_U * Nq] = twice(hu);
+      W[C::W_V * Nq] = twice(hv);
       W[C::W_BETA * Nq] = beta;
       W[C::W_LR * Nq] = log_fast(rho, op);
       W[C::W_LB * Nq] = log_fast<true>(beta, op);  // log of the reference's beta
@@ -371,7 +393,7 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
       P.U[1] = ax ? S[2] : S[1];
       P.U[2] = ax ? S[1] : S[2];
       P.U[3] = S[3];
-      const double rr = rcp(P.U[0]), hr = dmul(0.5, rr);
+      const double rr = rcp(P.U[0]), hr = half(rr);
       const double hn = dmul(P.U[1], hr), ht = dmul(P.U[2], hr);
       const double pe = dsub(P.U[3], dfma(P.U[1], hn, dmul(P.U[2], ht)));
       line_node(P, hn, ht, dmul(a.hgm1, pe), dmul(a.cws, rr));
@@ -382,7 +404,7 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
     // phi of the face between A (lower) and B with half wavespeed wv (signed)
     auto face = [&](const LineNode& A, const LineNode& B, double wv, int t) {
       const int f = f0 + fs * t;
-      PH[f] = dfma(-wv, dsub(B.U[0], A.U[0]), dmul(0.5, dadd(A.U[1], B.U[1])));
+      PH[f] = dfma(-wv, dsub(B.U[0], A.U[0]), half(dadd(A.U[1], B.U[1])));
       PH[cn * NF + f] = dfma(-wv, dsub(B.U[1], A.U[1]), dadd(A.fn, B.fn));
       PH[ct * NF + f] = dfma(-wv, dsub(B.U[2], A.U[2]), dadd(A.ft, B.ft));
       PH[3 * NF + f] = dfma(-wv, dsub(B.U[3], A.U[3]), dadd(A.fe, B.fe));

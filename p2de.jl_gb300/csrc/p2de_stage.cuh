@@ -121,21 +121,69 @@ struct Cfg {
 // U + dt rhsL, the low-order update (one form everywhere, so values agree bitwise)
 __device__ __forceinline__ double low_update(double u, double dt, double r) { return fma(dt, r, u); }
 
-// 1/x: for |x| in [2^-1022, 2^1022) (a normal reciprocal) two Newton-Raphson steps
-// y <- y + y (1 - x y) from the hardware's approximate reciprocal (rcp.approx.ftz.f64),
-// each residual formed by an FMA; the result is the correctly rounded 1/x unless 1/x lies
-// within about 2^-88 relative of a rounding tie (the same bits as __drcp_rn on 4M random
-// arguments), in 5 FP64 instructions against 6. Other x (0, subnormal, huge, inf, NaN) take
-// __drcp_rn.
+// 1/x and sqrt(x) with most of the work off the FP64 pipe, which issues one warp instruction
+// per 17-20 clocks and SM here: an FP32 approximation (2^-23) is refined to about 44 bits in
+// FP32 and integer arithmetic (24-30 instructions on pipes that otherwise issue in a tenth of
+// their slots), and one FP64 Newton-Raphson step y + y (1 - x y), or for the root the step
+// g + (x - g g) y/2 from g = x y, y ~ 1/sqrt(x), gives the correctly rounded result unless it
+// lies within about 2^-88 relative of a rounding tie. 2 and 3 FP64 operations, 36 and 52 SM
+// clocks a warp; two Newton steps from the hardware's 20-bit FP64 reciprocal take 4 and 71
+// clocks, CUDA's square root 9 and 145. Compared on 8.6e9 arguments over the whole range: the
+// bits of __dsqrt_rn always, those of __drcp_rn but for mantissas of 53 ones (a tie to 2^-106,
+// where the two-step form rounds down too).
+//
+// seed_value: the double (y0 + v 2^-44) 2^-k for a float y0 in [1/2, 1], |v| < 2^22 and
+// sub = k << 20.
+__device__ __forceinline__ double seed_value(float y0, int v, int sub) {
+  const unsigned b = (unsigned)__float_as_int(y0);
+  const unsigned long long y =
+      ((unsigned long long)((b >> 3) + (896u << 20)) << 32 | (b << 29)) + (unsigned long long)(long long)(v * 512);
+  return __hiloint2double((int)(y >> 32) - sub, (int)(unsigned)y);
+}
+// the 29 mantissa bits of a double below its leading 24, cut to 23, as a float in [0, 1) 2^s
+// for the float exponent bits eb = (127 + s) << 23
+__device__ __forceinline__ float low_bits(unsigned lo, int eb) {
+  return __fsub_rn(__int_as_float((int)((lo >> 6) & 0x7fffffu) | eb), __int_as_float(eb));
+}
+constexpr float kSeedMagic = 12582912.0f;  // 1.5 2^23: the low mantissa bits of x + this are x as an integer
+
+// 1/x for |x| in [2^-1021, 2^1021); other x take __drcp_rn
 __device__ __forceinline__ double rcp(double x) {
-  const unsigned long long a = (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffULL;
-  if (a - 0x0010000000000000ULL >= 0x7fc0000000000000ULL) return __drcp_rn(x);
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  double e = fma(-x, y, 1.0);
-  y = fma(y, e, y);
-  e = fma(-x, y, 1.0);
-  return fma(y, e, y);
+  const int hi = __double2hiint(x);
+  const unsigned lo = (unsigned)__double2loint(x);
+  if ((unsigned)((hi & 0x7fffffff) - 0x00200000) >= 0x7fa00000u) return __drcp_rn(x);
+  const float xh = __int_as_float((int)(__funnelshift_l(lo, (unsigned)hi, 3) & 0x7fffffu) | 0x3f800000);
+  const float xl = low_bits(lo, 0x3f800000);
+  float y0;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(xh));
+  float e = __fmaf_rn(-xh, y0, 1.0f);
+  e = __fmaf_rn(__fmul_rn(y0, -0x1p-23f), xl, e);  // 1 - x y0
+  const int v = __float_as_int(__fmaf_rn(__fmul_rn(y0, 0x1p44f), e, kSeedMagic)) - 0x4b400000;
+  double y = seed_value(y0, v, (hi & 0x7ff00000) - (1023 << 20));
+  y = __hiloint2double(__double2hiint(y) | (hi & (int)0x80000000), __double2loint(y));
+  return __fma_rn(y, __fma_rn(-x, y, 1.0), y);
+}
+
+// sqrt(x) for x in [2^-900, 2^900]; other x take __dsqrt_rn
+__device__ __forceinline__ double sqrt_rn(double x) {
+  const int hi = __double2hiint(x);
+  const unsigned lo = (unsigned)__double2loint(x);
+  if ((unsigned)(hi - (123 << 20)) >= (1800u << 20)) return __dsqrt_rn(x);
+  // x = m 4^k with m in [1, 4)
+  const int mb = (int)((__funnelshift_l(lo, (unsigned)hi, 3) & 0xffffffu) ^ 0x800000u) + 0x3f800000;
+  const float xh = __int_as_float(mb), xl = low_bits(lo, mb & 0x7f800000);
+  const int k20 = ((hi - (1023 << 20)) >> 1) & (int)0xfff00000;  // k << 20
+  float y0;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(xh));
+  const float th = __fmul_rn(y0, y0), tl = __fmaf_rn(y0, y0, -th);
+  float e = __fmaf_rn(-xh, th, 1.0f);
+  e = __fmaf_rn(-xh, tl, e);
+  e = __fmaf_rn(__fmul_rn(th, -0x1p-23f), xl, e);  // 1 - m y0^2
+  const int v = __float_as_int(__fmaf_rn(__fmul_rn(y0, 0x1p43f), e, kSeedMagic)) - 0x4b400000;
+  const double y = seed_value(y0, v, k20);
+  const double g = __dmul_rn(x, y);
+  const double h = __hiloint2double(__double2hiint(y) - (1 << 20), __double2loint(y));
+  return __fma_rn(__fma_rn(-g, g, x), h, g);
 }
 
 // Natural logarithm by the table-driven method of P. T. P. Tang ("Table-driven implementation
@@ -161,9 +209,12 @@ __device__ __forceinline__ double log_fast(double x, const OpTable& op) {
     k += 1;
   }
   const double m = __longlong_as_double(mb);
-  const double t = m + 0x1p44;  // m rounded to a multiple of 2^-8 in the low mantissa bits
-  const int j = (int)(__double_as_longlong(t) & 0x1ff);
-  const double F = t - 0x1p44;
+  // F = m rounded to a multiple of 2^-8, on the integer pipe: the exponent field is 1023 (m in
+  // [1, sqrt 2)) or 1022
+  const int mh = (int)(mb >> 32), sh = 13 - (mh >> 20 & 1);
+  const int Fh = ((mh >> (sh - 1)) + 1) >> 1;  // F in units of 2^-7 or 2^-8 above its binade
+  const double F = __hiloint2double(Fh << sh, 0);
+  const int j = Fh - (sh == 12 ? (0x3ff00000 >> 12) - 256 : (0x3fe00000 >> 13) - 128);
   const double* T = op.logtab[j - kLogTabLo];
   const double r = (m - F) * T[0];
   double q = fma(r, -1.0 / 6.0, 1.0 / 5.0);
@@ -211,7 +262,7 @@ __device__ __forceinline__ long long order_key(double x) {
 // gamma*(gamma-1) is one constant)
 __device__ __forceinline__ double wavespeed_r(const Gas<double>& g, double rr, double un, double E) {
   double pe = fma(-0.5, (un * un) * rr, E);
-  return fabs(un * rr) + sqrt((g.gamma * g.gm1) * pe * rr);
+  return fabs(un * rr) + sqrt_rn((g.gamma * g.gm1) * pe * rr);
 }
 
 // x with its sign flipped when sign < 0 (integer pipe): q + signed(x, s) is q + s*x for s = +-1
@@ -344,7 +395,7 @@ __device__ __forceinline__ double rhoe_quadratic_solve(const double* U, const do
   double l = 1.0;
   double disc = b * b - 4.0 * a * c;
   if (disc >= 0.0) {
-    double sq = sqrt(disc);
+    double sq = sqrt_rn(disc);
     double r2a = rcp(2.0 * a);
     double r1 = (-b + sq) * r2a;
     double r2 = (-b - sq) * r2a;
