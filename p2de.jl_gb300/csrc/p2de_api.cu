@@ -1009,9 +1009,20 @@ int p2de_ssp33_advance(p2de_solver* s, int64_t nsteps, double* t, int64_t* steps
   CK(cudaStreamSynchronize(s->stream));
   double steps0 = sc[S_STEPS];
   CK(cudaMemcpyAsync(s->scal + S_T, t, sizeof(double), cudaMemcpyHostToDevice, s->stream));
-  for (int64_t i = 0; i < nsteps; ++i) {
-    CK(cudaGraphLaunch(s->graph, s->stream));
-    s->launches += step_launches(s);
+  double now = sc[S_T] = *t, dt = 0.0;
+  const int per_step = step_launches(s);
+  for (int64_t left = nsteps; left > 0;) {
+    const int64_t n = steps_ahead(now, s->prm.T, dt, left);
+    for (int64_t i = 0; i < n; ++i) {
+      CK(cudaGraphLaunch(s->graph, s->stream));
+      s->launches += per_step;
+    }
+    left -= n;
+    CK(cudaMemcpyAsync(sc, s->scal, sizeof sc, cudaMemcpyDeviceToHost, s->stream));
+    CK(cudaStreamSynchronize(s->stream));
+    now = sc[S_T];
+    dt = sc[S_DT];
+    if (sc[S_DONE] != 0.0 || !(now < s->prm.T)) break;
   }
   CK(cudaMemcpyAsync(sc, s->scal, sizeof sc, cudaMemcpyDeviceToHost, s->stream));
   CK(cudaStreamSynchronize(s->stream));
@@ -1026,13 +1037,7 @@ int p2de_ssp33(p2de_solver* s, double* t_out, int64_t* steps_out, double* dt_las
   CK(cudaSetDevice(s->device));
   double t = s->prm.t0;
   int64_t total = 0;
-  int rc = P2DE_OK;
-  for (;;) {
-    int64_t done = 0;
-    rc = p2de_ssp33_advance(s, 64, &t, &done);
-    total += done;
-    if (rc != P2DE_OK || done < 64 || !(t < s->prm.T)) break;
-  }
+  const int rc = p2de_ssp33_advance(s, INT64_MAX, &t, &total);
   if (t_out) *t_out = t;
   if (steps_out) *steps_out = total;
   if (s->line) {

@@ -2002,15 +2002,26 @@ int run_steps(LineSolve* L, double* t, int64_t nsteps, double ts_out[TS_N], std:
       if (g) cudaGraphDestroy(g);
     }
   }
-  for (int64_t i = 0; i < nsteps && e == cudaSuccess; ++i) {
-    if (L->graph) {
-      e = cudaGraphLaunch(L->graph, L->stream);
-      L->launches += line_step_launches(L);
-    } else {
-      e = enqueue_step(L);
+  const int per_step = line_step_launches(L);
+  double now = *t, dt = 0.0;
+  int64_t left = nsteps;
+  do {
+    const int64_t n = steps_ahead(now, L->prm.T, dt, left);
+    for (int64_t i = 0; i < n && e == cudaSuccess; ++i) {
+      if (L->graph) {
+        e = cudaGraphLaunch(L->graph, L->stream);
+        L->launches += per_step;
+      } else {
+        e = enqueue_step(L);
+      }
     }
-  }
-  if (e == cudaSuccess) e = cudaMemcpyAsync(ts_out, L->ts, sizeof(double) * TS_N, cudaMemcpyDeviceToHost, L->stream);
+    left -= n;
+    if (e == cudaSuccess) e = cudaMemcpyAsync(ts_out, L->ts, sizeof(double) * TS_N, cudaMemcpyDeviceToHost, L->stream);
+    if (e != cudaSuccess || left == 0) break;
+    e = cudaStreamSynchronize(L->stream);
+    now = ts_out[TS_T];
+    dt = ts_out[TS_DT];
+  } while (e == cudaSuccess && ts_out[TS_DONE] == 0.0 && now < L->prm.T);
   if (e != cudaSuccess) {
     err = std::string("line steps: ") + cudaGetErrorString(e);
     return P2DE_ERR_CUDA;
