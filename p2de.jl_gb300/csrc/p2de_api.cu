@@ -615,8 +615,12 @@ int p2de_initialize_DG(const p2de_param* prm, const p2de_mesh* mesh, int device,
                       own_faces(mesh->mapW, mesh->nW, mesh->mapP) && own_faces(mesh->mapS, mesh->nS, mesh->mapP);
   s->flux = flags_for(s, 2, false, false) & F_FLUX;
   if (s->flux) {  // its own shared-memory layout
-    s->geo.elems_per_block = s->geo.elems_per_block_flux;
+    const FluxShape shape = flux_shape(s->N1D, s->K, s->geo.elems_per_block_flux,
+                                       flags_for(s, 2, false, false) & kExtFlags);
+    s->geo.elems_per_block = shape.epb;
     s->geo.elems_per_block_max = s->geo.elems_per_block_max_flux;
+    s->base.threads = shape.threads;
+    s->base.split = shape.split;
   }
 #define DA(ptr, cnt)                                                                     \
   do {                                                                                   \
@@ -675,7 +679,6 @@ int p2de_initialize_DG(const p2de_param* prm, const p2de_mesh* mesh, int device,
   StageArgs& a = s->base;
   a.K = s->K;
   a.epb = s->geo.elems_per_block;
-  if (s->flux) a.threads = flux_threads(s->K, a.epb);
   a.ops = table_of(s);
   a.Uq = s->Uq;
   a.resW = s->resW;
@@ -1024,8 +1027,6 @@ int p2de_ssp33_advance(p2de_solver* s, int64_t nsteps, double* t, int64_t* steps
     dt = sc[S_DT];
     if (sc[S_DONE] != 0.0 || !(now < s->prm.T)) break;
   }
-  CK(cudaMemcpyAsync(sc, s->scal, sizeof sc, cudaMemcpyDeviceToHost, s->stream));
-  CK(cudaStreamSynchronize(s->stream));
   rc = check_status(s);
   *t = sc[S_T];
   if (steps_done) *steps_done = (int64_t)(sc[S_STEPS] - steps0);

@@ -57,6 +57,7 @@ struct StageArgs {
   int layout;
   // threads per block of stage kernel A (a multiple of 32 up to Cfg::THREADS; 0: Cfg::THREADS)
   int threads;
+  int split;  // flux form: lines spread over the block (flux_shape)
   const OpTable* ops;
   double* Uq;
   double* resW;
@@ -135,7 +136,6 @@ inline bool flux_form(int flags, int N, double zerotol, bool own_boundaries, boo
          !((flags & F_SHOCK) && (flags & F_REF_SEM)) && !acc32 && own_boundaries && zerotol < 0.999999 / ((double)N * (N + 1));
 }
 
-// StageArgs shock-capture constants of update_blending_factor! (shock_capture.jl:123-126)
 // Steps to launch before looking at the device's time again: enough to reach T at the last
 // step size, so that a run which ends (or fails) earlier than nsteps does not replay the step
 // as no-ops, seven launches each (the 5x5 vortex solve takes 8 steps of the 64 that
@@ -148,6 +148,7 @@ inline int64_t steps_ahead(double t, double T, double dt, int64_t left) {
   return left < n ? left : n;
 }
 
+// StageArgs shock-capture constants of update_blending_factor! (shock_capture.jl:123-126)
 inline void set_shock_capture(StageArgs& a, int N, double sc_a, double sc_c) {
   const double TN = sc_a * std::pow(10.0, -sc_c * std::pow((double)(N + 1), 0.25));
   const double alphaE0 = 0.0001;

@@ -46,6 +46,12 @@ __device__ __forceinline__ double scale_exponent(double x, int step) {
 __device__ __forceinline__ double half(double x) { return scale_exponent(x, -0x00100000); }
 __device__ __forceinline__ double twice(double x) { return scale_exponent(x, 0x00100000); }
 
+__device__ __forceinline__ bool negative(double x) { return __double2hiint(x) < 0; }
+// |x| > t (t > 0), x not NaN, by the bits
+__device__ __forceinline__ bool magnitude_above(double x, double t) {
+  const long long b = __double_as_longlong(x) & 0x7fffffffffffffffLL;
+  return b > __double_as_longlong(t) && b <= 0x7ff0000000000000LL;
+}
 // > 0 and not NaN, by the bits
 __device__ __forceinline__ bool positive_bits(double x) {
   const long long b = __double_as_longlong(x);
@@ -82,7 +88,8 @@ struct FluxCfg {
   static constexpr int W_HU = 0, W_HV = 1, W_U = 2, W_V = 3, W_BETA = 4, W_LR = 5, W_LB = 6, W_PH = 7, W_CRR = 8,
                        W_IND = 9, W_EN = 10;
   static constexpr int W_UL = 0, W_LRHOE = 4, W_LRHO = 5, W_URHO = 6, W_THR = 7, W_QC = 8, W_EV = 10;
-  template <bool EXT>
+  static constexpr int NPH = NL * PPL;
+  template <bool EXT, bool SPLIT = false>
   struct Lay {
     static constexpr int O_R = O_W + (EXT ? 14 : 12) * Nq;  // 4 Nq: rhsL; before that CFL sums (0, 1)
     static constexpr int O_PH = O_R + 4 * Nq;               // 4 NF: low-order (then limited) fluxes
@@ -90,16 +97,24 @@ struct FluxCfg {
     static constexpr int O_L = O_DF + 4 * NF;               // NF: factors
     // smoothness factor of the relaxed bounds, 2 flags of the entropy phase, blending factor
     static constexpr int O_X = O_L + NF;
-    static constexpr int PE = O_X + 4;
+    // SPLIT: pair fluxes, along-axis node values (normal, tangential and energy half flux, half
+    // wavespeed; per direction), half wavespeeds of the faces
+    static constexpr int O_SF = O_X + 4;
+    static constexpr int O_SN = O_SF + 4 * NPH;
+    static constexpr int O_SW = O_SN + 8 * Nq;
+    static constexpr int PE = SPLIT ? O_SW + NF : O_X + 4;
   };
   // plus the list of faces whose bounds need solves (and, EXT, the list of bisections)
-  template <bool EXT>
+  template <bool EXT, bool SPLIT = false>
   static constexpr size_t smem(int e) {
-    return sizeof(double) * Lay<EXT>::PE * e + sizeof(int) * ((size_t)NF * e + 4 + (EXT ? 2 * (size_t)NF * e : 0));
+    return sizeof(double) * Lay<EXT, SPLIT>::PE * e + sizeof(int) * ((size_t)NF * e + 4 + (EXT ? 2 * (size_t)NF * e : 0));
   }
   static constexpr int E_MAX_RAW =
       (int)((224 * 1024 - 64) / (sizeof(double) * Lay<true>::PE + sizeof(int) * 3 * NF));
   static constexpr int E_MAX = E_MAX_RAW < 32 ? E_MAX_RAW : 32;
+  static constexpr int E_SPLIT_RAW =
+      (int)((224 * 1024 - 64) / (sizeof(double) * Lay<false, true>::PE + sizeof(int) * NF));
+  static constexpr int E_SPLIT_MAX = E_SPLIT_RAW < 32 ? E_SPLIT_RAW : 32;
   static_assert(E <= E_MAX, "flux layout");
 };
 
@@ -220,12 +235,176 @@ __device__ __forceinline__ void line_node(LineNode& q, double hn, double ht, dou
   q.wh = dadd(fabs(hn), sqrt_rn(dmul(pe, crr)));
 }
 
+// One line of an element: its places in the element's shared memory and the pieces of its
+// fluxes. Components of states and fluxes here are (rho, normal, tangential, E).
+//
+// Two layouts call them, with the same operations per value and so the same bits. On large
+// meshes one thread takes a whole line: the fewest FP64 instructions, all lanes busy. An SM
+// quarter issues one FP64 warp instruction per 64 clocks and holds no second one in flight
+// (measured: 64 clocks a dependent chain, with 1 to 8 chains in a warp), so on small meshes,
+// where an SM has few warps, a line's chain of ~300 instructions is the stage's duration;
+// SPLIT spreads the pairs, boundary faces, node values and sums over the block's warps.
+template <int N1D, class Y>
+struct FluxLine {
+  using C = FluxCfg<N1D>;
+  static constexpr int n = C::n, Nq = C::Nq, Nfp = C::Nfp, NSF = C::NSF, NF = C::NF;
+  const StageArgs& a;
+  const OpTable& op;
+  double* base;
+  const int k, ax, l;
+  const double t_now, gd;
+  const int sg;     // the sign of f_bar's unit
+  const bool visc;  // the reference adds the viscosity of an x pair only when |S0x| > 1e-10 (:156-163)
+  const int q0, qs;  // nodes q0 + qs i
+  const int f0, fs;  // faces f0 + fs t
+  double *PH, *DF;
+
+  __device__ __forceinline__ FluxLine(const StageArgs& a_, const OpTable& op_, double* base_, int k_, int ax_, int l_,
+                                      double t_)
+      : a(a_), op(op_), base(base_), k(k_), ax(ax_), l(l_), t_now(t_), gd(a_.geom[5 * (size_t)k_ + (ax_ ? 4 : 1)]),
+        sg(negative(gd) ? -1 : 1),
+        visc(ax_ == 1 || magnitude_above(dmul(gd, op_.lp_S[l_ * (n - 1)]), 1e-10)),
+        q0(ax_ ? l_ : n * l_), qs(ax_ ? n : 1), f0(ax_ ? NSF + l_ : (n + 1) * l_), fs(ax_ ? n : 1),
+        PH(base_ + Y::O_PH), DF(base_ + Y::O_DF) {}
+
+  // the array component of line component q
+  __device__ __forceinline__ int comp(int q) const { return q == 1 ? 1 + ax : q == 2 ? 2 - ax : q; }
+
+  __device__ __forceinline__ void load(int i, LineNode& q) const {
+    const double* U = base + C::O_U + q0 + qs * i;
+    const double* W = base + C::O_W + q0 + qs * i;
+    q.U[0] = U[0];
+    q.U[1] = U[(1 + ax) * Nq];
+    q.U[2] = U[(2 - ax) * Nq];
+    q.U[3] = U[3 * Nq];
+    line_node(q, W[ax * Nq], W[(1 - ax) * Nq], W[C::W_PH * Nq], W[C::W_CRR * Nq]);
+  }
+
+  // the exterior state at boundary face `side` of the line (0 low, 1 high) and its values; off:
+  // the high-order flux has no dissipation there
+  __device__ __forceinline__ void exterior(int side, const LineNode& own, LineNode& P, bool& off) const {
+    const size_t fk = (size_t)k * Nfp + (2 * ax + side) * n + l;
+    const int lin = a.nbr[fk], code = a.bc[fk];
+    double S[4];
+    if (code == BC_INTERIOR) {
+      const int kP = lin / Nfp, iP = lin % Nfp, sP = iP / n, tP = iP % n;
+      const int qP = sP == 0 ? n * tP : sP == 1 ? (n - 1) + n * tP : sP == 2 ? tP : tP + n * (n - 1);
+      const double* s = a.Uq + ((size_t)kP * Nq + qP) * 4;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) S[c] = __ldg(s + c);
+    } else if (code == BC_INFLOW) {
+      const double* iv = a.Ival + 4 * (size_t)a.bcidx[fk];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) S[c] = iv[c];
+    } else if (code == BC_SHOCK) {
+      const double* xy = a.xyS + 2 * (size_t)a.bcidx[fk];
+      const bool post = xy[0] < a.shock_x0 + (xy[1] + a.shock_speed * t_now) * a.shock_inv_slope;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) S[c] = post ? a.shock_post[c] : a.shock_pre[c];
+    } else {  // outflow: the own state; wall: the own state reflected along the axis
+      const double mn = code == BC_WALL ? -own.U[1] : own.U[1];
+      S[0] = own.U[0];
+      S[1] = ax ? own.U[2] : mn;
+      S[2] = ax ? mn : own.U[2];
+      S[3] = own.U[3];
+    }
+    P.U[0] = S[0];
+    P.U[1] = ax ? S[2] : S[1];
+    P.U[2] = ax ? S[1] : S[2];
+    P.U[3] = S[3];
+    const double rr = rcp(P.U[0]), hr = half(rr);
+    const double hn = dmul(P.U[1], hr), ht = dmul(P.U[2], hr);
+    const double pe = dsub(P.U[3], dfma(P.U[1], hn, dmul(P.U[2], ht)));
+    line_node(P, hn, ht, dmul(a.hgm1, pe), dmul(a.cws, rr));
+    // a boundary face's wavespeed is the own one (its mapP is itself)
+    if (code != BC_INTERIOR) P.wh = own.wh;
+    off = code == BC_INFLOW || code == BC_OUTFLOW || code == BC_SHOCK;
+  }
+
+  // phi of face t between A (lower) and B with half wavespeed w
+  __device__ __forceinline__ void face(const LineNode& A, const LineNode& B, double w, int t) const {
+    const double wv = visc || t == 0 || t == n ? signed_by(w, sg) : 0.0;
+    double* ph = PH + f0 + fs * t;
+    ph[0] = dfma(-wv, dsub(B.U[0], A.U[0]), half(dadd(A.U[1], B.U[1])));
+    ph[(1 + ax) * NF] = dfma(-wv, dsub(B.U[1], A.U[1]), dadd(A.fn, B.fn));
+    ph[(2 - ax) * NF] = dfma(-wv, dsub(B.U[2], A.U[2]), dadd(A.ft, B.ft));
+    ph[3 * NF] = dfma(-wv, dsub(B.U[3], A.U[3]), dadd(A.fe, B.fe));
+  }
+  // high minus low order at a boundary face: the dissipation where the high-order flux has none
+  __device__ __forceinline__ void face_diff(const LineNode& A, const LineNode& B, double w, bool off, int t) const {
+    const double wv = signed_by(w, sg);
+    double* df = DF + f0 + fs * t;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) df[comp(q) * NF] = off ? dmul(wv, dsub(B.U[q], A.U[q])) : 0.0;
+  }
+  // the surface terms B f* of boundary face `side` for p2de_get_field, from phi and dF
+  __device__ __forceinline__ void debug_surface(int side) const {
+    const int f = f0 + fs * (side ? n : 0);
+    const double gw = gd * op.w1D[l] * (side ? 1.0 : -1.0);
+    const size_t g = ((size_t)k * Nfp + (2 * ax + side) * n + l) * 8;
+    for (int c = 0; c < 4; ++c) {
+      a.BFL[g + 4 * ax + c] = gw * PH[c * NF + f];
+      a.BFH[g + 4 * ax + c] = gw * (PH[c * NF + f] + DF[c * NF + f]);
+      a.BFL[g + 4 - 4 * ax + c] = a.BFH[g + 4 - 4 * ax + c] = 0.0;
+    }
+  }
+  // node i's share of the CFL sum along this line: the half wavespeeds of its two faces
+  __device__ __forceinline__ void cfl_sum(int i, double wl, double wr) const {
+    base[Y::O_R + ax * Nq + q0 + qs * i] = dadd(wl, wr);
+  }
+
+  // the two-point flux of line nodes i > j; in FP32 (TH = float) already times its coefficient
+  // and converted
+  template <typename TH>
+  __device__ __forceinline__ void pair(const Gas<float>& gf, int i, int j, double* F) const {
+    const int mi = q0 + qs * i, mj = q0 + qs * j;
+    if constexpr (sizeof(TH) == 8) {
+      PairState qi, qj;
+      pstate(mi, qi);
+      pstate(mj, qj);
+      fS_line(a.rgm1, qj, qi, &F[0], &F[2], &F[1], &F[3]);
+    } else {
+      const float* Wf = reinterpret_cast<const float*>(base + C::O_W + 4 * Nq);
+      const float UJ[4] = {Wf[mj], Wf[Nq + mj], Wf[2 * Nq + mj], Wf[3 * Nq + mj]};
+      const float UI[4] = {Wf[mi], Wf[Nq + mi], Wf[2 * Nq + mi], Wf[3 * Nq + mi]};
+      const float c = op.hpcf[(ax * n + l) * C::PPL + i * (i - 1) / 2 + j];
+      float G[4];
+      fS_f32_axis(gf, UI, UJ, ax, G);
+      F[0] = (double)__fmul_rn(c, G[0]);
+      F[1] = (double)__fmul_rn(c, ax ? G[2] : G[1]);
+      F[2] = (double)__fmul_rn(c, ax ? G[1] : G[2]);
+      F[3] = (double)__fmul_rn(c, G[3]);
+    }
+  }
+  // suffix sum s over the pairs (i.., j) of one component, started at i = n - 1
+  template <typename TH>
+  __device__ __forceinline__ double suffix(int i, int j, double F, double s) const {
+    if constexpr (sizeof(TH) == 8) {
+      const double c = op.hpc[(ax * n + l) * C::PPL + i * (i - 1) / 2 + j];
+      return i == n - 1 ? dmul(c, F) : dfma(c, F, s);
+    } else {
+      return i == n - 1 ? F : dadd(s, F);
+    }
+  }
+  __device__ __forceinline__ void pstate(int m, PairState& q) const {
+    const double* W = base + C::O_W + m;
+    q.rho = base[C::O_U + m];
+    q.vn = W[(C::W_U + ax) * Nq];
+    q.vt = W[(C::W_V - ax) * Nq];
+    q.hn = W[ax * Nq];
+    q.ht = W[(1 - ax) * Nq];
+    q.beta = W[C::W_BETA * Nq];
+    q.lr = W[C::W_LR * Nq];
+    q.lb = W[C::W_LB * Nq];
+  }
+};
+
 // The body for the elements k0 .. k0 + epb - 1 of the solve `a`; early returns are uniform
 // over the block.
-template <int N1D, typename TH, bool EXT>
+template <int N1D, typename TH, bool EXT, bool SPLIT = false>
 __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* sm) {
   using C = FluxCfg<N1D>;
-  using Y = typename C::template Lay<EXT>;
+  using Y = typename C::template Lay<EXT, SPLIT>;
   constexpr int n = C::n, Nq = C::Nq, Nfp = C::Nfp, NL = C::NL, NSF = C::NSF, NF = C::NF, NI = C::NI, PE = Y::PE;
   constexpr bool F32 = sizeof(TH) == 4;
   if (a.scal[S_DONE] != 0.0) return;
@@ -343,189 +522,55 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
     __syncthreads();
   }
 
-  // ---- line phase: one thread per (element, direction, tangential node)
+  // ---- lines: one thread per (element, direction, tangential node), or SPLIT (FluxLine)
   const bool low_only = flags & F_LOW_ONLY;
+  const bool cfl = flags & F_CFL;
   const Gas<float> gf{a.gasf[0], a.gasf[1], a.gasf[2]};
-  for (int w = tid; w < Ke * NL; w += bs) {
-    const int e = w / NL, r = w % NL, ax = r / n, l = r % n, k = k0 + e;
-    double* base = sm + e * PE;
-    const double gd = a.geom[5 * (size_t)k + (ax ? 4 : 1)];
-    const int sg = gd < 0.0 ? -1 : 1;  // the sign of f_bar's unit
-    // the reference adds the viscosity of an x pair only when |S0x| > 1e-10 (:156-163)
-    const bool visc = ax == 1 || fabs(dmul(gd, op.lp_S[l * (n - 1)])) > 1e-10;
-    const int q0 = ax ? l : n * l, qs = ax ? n : 1;          // nodes q0 + qs i
-    const int f0 = ax ? NSF + l : (n + 1) * l, fs = ax ? n : 1;  // faces f0 + fs t
-    const double* Un = base + C::O_U + (1 + ax) * Nq;  // normal momentum
-    const double* Ut = base + C::O_U + (2 - ax) * Nq;
-    const double* U0 = base + C::O_U;
-    const double* W = base + C::O_W;
-    double* PH = base + Y::O_PH;
-    double* DF = base + Y::O_DF;
-    const int cn = 1 + ax, ct = 2 - ax;
-    // the exterior state at boundary face `side` of the line (0 low, 1 high) and its values
-    auto exterior = [&](int side, const LineNode& own, LineNode& P, bool& off) {
-      const int f = (2 * ax + side) * n + l;
-      const size_t fk = (size_t)k * Nfp + f;
-      const int lin = a.nbr[fk], code = a.bc[fk];
-      double S[4];
-      if (code == BC_INTERIOR) {
-        const int kP = lin / Nfp, iP = lin % Nfp, sP = iP / n, tP = iP % n;
-        const int qP = sP == 0 ? n * tP : sP == 1 ? (n - 1) + n * tP : sP == 2 ? tP : tP + n * (n - 1);
-        const double* s = a.Uq + ((size_t)kP * Nq + qP) * 4;
+  if constexpr (!SPLIT) {
+    for (int w = tid; w < Ke * NL; w += bs) {
+      const int e = w / NL, r = w % NL;
+      FluxLine<N1D, Y> ln(a, op, sm + e * PE, k0 + e, r / n, r % n, t_now);
+      {
+        LineNode A, B, P;
+        bool off;
+        ln.load(0, A);
+        ln.exterior(0, A, P, off);
+        double wl = max_nonneg_bits(P.wh, A.wh);
+        ln.face(P, A, wl, 0);
+        ln.face_diff(P, A, wl, off, 0);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) S[c] = __ldg(s + c);
-      } else if (code == BC_INFLOW) {
-        const double* iv = a.Ival + 4 * (size_t)a.bcidx[fk];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) S[c] = iv[c];
-      } else if (code == BC_SHOCK) {
-        const double* xy = a.xyS + 2 * (size_t)a.bcidx[fk];
-        const bool post = xy[0] < a.shock_x0 + (xy[1] + a.shock_speed * t_now) * a.shock_inv_slope;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) S[c] = post ? a.shock_post[c] : a.shock_pre[c];
-      } else {  // outflow: the own state; wall: the own state reflected along the axis
-        S[0] = own.U[0];
-        S[cn] = code == BC_WALL ? -own.U[1] : own.U[1];
-        S[ct] = own.U[2];
-        S[3] = own.U[3];
+        for (int i = 1; i < n; ++i) {
+          ln.load(i, B);
+          const double wr = max_nonneg_bits(A.wh, B.wh);
+          ln.face(A, B, wr, i);
+          if (cfl) ln.cfl_sum(i - 1, wl, wr);
+          wl = wr;
+          A = B;
+        }
+        ln.exterior(1, A, P, off);
+        const double wr = max_nonneg_bits(P.wh, A.wh);
+        ln.face(A, P, wr, n);
+        ln.face_diff(A, P, wr, off, n);
+        if (cfl) ln.cfl_sum(n - 1, wl, wr);
       }
-      P.U[0] = S[0];
-      P.U[1] = ax ? S[2] : S[1];
-      P.U[2] = ax ? S[1] : S[2];
-      P.U[3] = S[3];
-      const double rr = rcp(P.U[0]), hr = half(rr);
-      const double hn = dmul(P.U[1], hr), ht = dmul(P.U[2], hr);
-      const double pe = dsub(P.U[3], dfma(P.U[1], hn, dmul(P.U[2], ht)));
-      line_node(P, hn, ht, dmul(a.hgm1, pe), dmul(a.cws, rr));
-      // a boundary face's wavespeed is the own one (its mapP is itself)
-      if (code != BC_INTERIOR) P.wh = own.wh;
-      off = code == BC_INFLOW || code == BC_OUTFLOW || code == BC_SHOCK;
-    };
-    // phi of the face between A (lower) and B with half wavespeed wv (signed)
-    auto face = [&](const LineNode& A, const LineNode& B, double wv, int t) {
-      const int f = f0 + fs * t;
-      PH[f] = dfma(-wv, dsub(B.U[0], A.U[0]), half(dadd(A.U[1], B.U[1])));
-      PH[cn * NF + f] = dfma(-wv, dsub(B.U[1], A.U[1]), dadd(A.fn, B.fn));
-      PH[ct * NF + f] = dfma(-wv, dsub(B.U[2], A.U[2]), dadd(A.ft, B.ft));
-      PH[3 * NF + f] = dfma(-wv, dsub(B.U[3], A.U[3]), dadd(A.fe, B.fe));
-    };
-    // high minus low order at a boundary face: the dissipation where the high-order flux has none
-    auto face_diff = [&](const LineNode& A, const LineNode& B, double wv, bool off, int t) {
-      const int f = f0 + fs * t;
-      DF[f] = off ? dmul(wv, dsub(B.U[0], A.U[0])) : 0.0;
-      DF[cn * NF + f] = off ? dmul(wv, dsub(B.U[1], A.U[1])) : 0.0;
-      DF[ct * NF + f] = off ? dmul(wv, dsub(B.U[2], A.U[2])) : 0.0;
-      DF[3 * NF + f] = off ? dmul(wv, dsub(B.U[3], A.U[3])) : 0.0;
-    };
-    // the surface terms B f* of face `side` for p2de_get_field, from phi and dF as just formed
-    auto debug_surface = [&](int side) {
-      const int f = f0 + fs * (side ? n : 0);
-      const double gw = gd * op.w1D[l] * (side ? 1.0 : -1.0);
-      const size_t g = ((size_t)k * Nfp + (2 * ax + side) * n + l) * 8;
-      for (int c = 0; c < 4; ++c) {
-        a.BFL[g + 4 * ax + c] = gw * PH[c * NF + f];
-        a.BFH[g + 4 * ax + c] = gw * (PH[c * NF + f] + DF[c * NF + f]);
-        a.BFL[g + 4 - 4 * ax + c] = a.BFH[g + 4 - 4 * ax + c] = 0.0;
+      if (low_only) continue;
+      if (flags & F_WRITE_DEBUG) {
+        ln.debug_surface(0);
+        ln.debug_surface(1);
       }
-    };
-    auto load = [&](int i, LineNode& q) {
-      const int m = q0 + qs * i;
-      q.U[0] = U0[m];
-      q.U[1] = Un[m];
-      q.U[2] = Ut[m];
-      q.U[3] = U0[3 * Nq + m];
-      line_node(q, W[ax * Nq + m], W[(1 - ax) * Nq + m], W[C::W_PH * Nq + m], W[C::W_CRR * Nq + m]);
-    };
-    {
-      LineNode A, B, P;
-      bool off;
-      load(0, A);
-      exterior(0, A, P, off);
-      double wl = max_nonneg_bits(P.wh, A.wh);
-      face(P, A, signed_by(wl, sg), 0);
-      face_diff(P, A, signed_by(wl, sg), off, 0);
-#pragma unroll
-      for (int i = 1; i < n; ++i) {
-        load(i, B);
-        const double wr = max_nonneg_bits(A.wh, B.wh);
-        face(A, B, visc ? signed_by(wr, sg) : 0.0, i);
-        if (flags & F_CFL) base[Y::O_R + ax * Nq + q0 + qs * (i - 1)] = dadd(wl, wr);
-        wl = wr;
-        A = B;
-      }
-      exterior(1, A, P, off);
-      const double wr = max_nonneg_bits(P.wh, A.wh);
-      face(A, P, signed_by(wr, sg), n);
-      face_diff(A, P, signed_by(wr, sg), off, n);
-      if (flags & F_CFL) base[Y::O_R + ax * Nq + q0 + qs * (n - 1)] = dadd(wl, wr);
-    }
-    if (low_only) continue;
-    if (flags & F_WRITE_DEBUG) {
-      debug_surface(0);
-      debug_surface(1);
-    }
-    // high order: for j ascending, the suffix sums over i of c_ij fS(i, j), added to face i
-    const int p0 = (ax * n + l) * C::PPL;
-    if constexpr (!F32) {
+      // high order: for j ascending, the suffix sums over i of c_ij fS(i, j), added to face i
       double acc[4][n];
-      auto pstate = [&](int i, PairState& q) {
-        const int m = q0 + qs * i;
-        q.rho = U0[m];
-        q.vn = W[(C::W_U + ax) * Nq + m];
-        q.vt = W[(C::W_V - ax) * Nq + m];
-        q.hn = W[ax * Nq + m];
-        q.ht = W[(1 - ax) * Nq + m];
-        q.beta = W[C::W_BETA * Nq + m];
-        q.lr = W[C::W_LR * Nq + m];
-        q.lb = W[C::W_LB * Nq + m];
-      };
 #pragma unroll
       for (int j = 0; j < n - 1; ++j) {
-        PairState qj;
-        pstate(j, qj);
         double s[4];
 #pragma unroll
         for (int i = n - 1; i > j; --i) {
-          PairState qi;
-          pstate(i, qi);
-          const double c = op.hpc[p0 + i * (i - 1) / 2 + j];
           double F[4];
-          fS_line(a.rgm1, qj, qi, &F[0], &F[2], &F[1], &F[3]);
+          ln.template pair<TH>(gf, i, j, F);
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
-            s[q] = i == n - 1 ? dmul(c, F[q]) : dfma(c, F[q], s[q]);
+            s[q] = ln.template suffix<TH>(i, j, F[q], s[q]);
             acc[q][i] = j == 0 ? s[q] : dadd(acc[q][i], s[q]);
-          }
-        }
-      }
-#pragma unroll
-      for (int t = 1; t < n; ++t) {
-        const int f = f0 + fs * t;
-        DF[f] = dsub(acc[0][t], PH[f]);
-        DF[cn * NF + f] = dsub(acc[1][t], PH[cn * NF + f]);
-        DF[ct * NF + f] = dsub(acc[2][t], PH[ct * NF + f]);
-        DF[3 * NF + f] = dsub(acc[3][t], PH[3 * NF + f]);
-      }
-    } else {
-      const float* Wf = reinterpret_cast<const float*>(base + C::O_W + 4 * Nq);
-      // FP32 two-point fluxes, their terms converted and summed in FP64
-      double sd[4], ad[4][n];
-#pragma unroll
-      for (int j = 0; j < n - 1; ++j) {
-        const int mj = q0 + qs * j;
-        const float UJ[4] = {Wf[mj], Wf[Nq + mj], Wf[2 * Nq + mj], Wf[3 * Nq + mj]};
-#pragma unroll
-        for (int i = n - 1; i > j; --i) {
-          const int mi = q0 + qs * i;
-          const float UI[4] = {Wf[mi], Wf[Nq + mi], Wf[2 * Nq + mi], Wf[3 * Nq + mi]};
-          const float c = op.hpcf[p0 + i * (i - 1) / 2 + j];
-          float F[4];
-          fS_f32_axis(gf, UI, UJ, ax, F);
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const double x = (double)__fmul_rn(c, F[q]);
-            sd[q] = i == n - 1 ? x : dadd(sd[q], x);
-            ad[q][i] = j == 0 ? sd[q] : dadd(ad[q][i], sd[q]);
           }
         }
       }
@@ -533,12 +578,100 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
       for (int t = 1; t < n; ++t)
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          const int f = q * NF + f0 + fs * t;
-          DF[f] = dsub(ad[q][t], PH[f]);
+          const int f = ln.comp(q) * NF + ln.f0 + ln.fs * t;
+          ln.DF[f] = dsub(acc[q][t], ln.PH[f]);
         }
     }
+    __syncthreads();
+  } else {
+    // the same operations spread over more threads: (element, pair) fluxes, boundary faces and
+    // along-axis node values, each in whole warps; then (element, line, component) sums
+    const int np = low_only ? 0 : Ke * NL * C::PPL, nb = Ke * Nfp, nn = Ke * 2 * Nq;
+    const int p32 = (np + 31) & ~31, b32 = (nb + 31) & ~31;
+    for (int w = tid; w < p32 + b32 + nn; w += bs) {
+      if (w < p32) {
+        if (w >= np) continue;
+        const int e = w / (NL * C::PPL), r = w % (NL * C::PPL), lr = r / C::PPL, pp = r % C::PPL;
+        double* base = sm + e * PE;
+        FluxLine<N1D, Y> ln(a, op, base, k0 + e, lr / n, lr % n, t_now);
+        int i = 1;  // pair pp = i (i - 1) / 2 + j
+        while (i * (i + 1) / 2 <= pp) ++i;
+        double F[4];
+        ln.template pair<TH>(gf, i, pp - i * (i - 1) / 2, F);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) base[Y::O_SF + q * C::NPH + r] = F[q];
+      } else if (w < p32 + b32) {
+        const int v = w - p32;
+        if (v >= nb) continue;
+        const int e = v / Nfp, side = (v % Nfp) / NL, lr = v % NL;
+        double* base = sm + e * PE;
+        FluxLine<N1D, Y> ln(a, op, base, k0 + e, lr / n, lr % n, t_now);
+        LineNode A, P;
+        bool off;
+        ln.load(side ? n - 1 : 0, A);
+        ln.exterior(side, A, P, off);
+        const double wv = max_nonneg_bits(P.wh, A.wh);
+        const int t = side ? n : 0;
+        ln.face(side ? A : P, side ? P : A, wv, t);
+        ln.face_diff(side ? A : P, side ? P : A, wv, off, t);
+        if (cfl) base[Y::O_SW + ln.f0 + ln.fs * t] = wv;
+        if (!low_only && (flags & F_WRITE_DEBUG)) ln.debug_surface(side);
+      } else {
+        const int v = w - p32 - b32, e = v / (2 * Nq), r = v % (2 * Nq), ax = r / Nq, m = r % Nq;
+        double* base = sm + e * PE;
+        const double* W = base + C::O_W;
+        LineNode A;
+        A.U[1] = base[C::O_U + (1 + ax) * Nq + m];
+        A.U[3] = base[C::O_U + 3 * Nq + m];
+        line_node(A, W[ax * Nq + m], W[(1 - ax) * Nq + m], W[C::W_PH * Nq + m], W[C::W_CRR * Nq + m]);
+        double* N = base + Y::O_SN + ax * 4 * Nq + m;
+        N[0] = A.fn;
+        N[Nq] = A.ft;
+        N[2 * Nq] = A.fe;
+        N[3 * Nq] = A.wh;
+      }
+    }
+    __syncthreads();
+    for (int w = tid; w < Ke * NL * 4; w += bs) {
+      const int e = w / (NL * 4), lr = w % (NL * 4) / 4, q = w % 4;
+      double* base = sm + e * PE;
+      FluxLine<N1D, Y> ln(a, op, base, k0 + e, lr / n, lr % n, t_now);
+      // the interior faces' low-order fluxes of component q (FluxLine::face, one component)
+      const double* N = base + Y::O_SN + ln.ax * 4 * Nq;
+      const double* Uq = base + C::O_U + ln.comp(q) * Nq;
+      const double* Fq = q == 0 ? base + C::O_U + (1 + ln.ax) * Nq : N + (q - 1) * Nq;
+      double* PH = ln.PH + ln.comp(q) * NF + ln.f0;
+      double* DF = ln.DF + ln.comp(q) * NF + ln.f0;
+      double uA = Uq[ln.q0], fA = Fq[ln.q0], wA = N[3 * Nq + ln.q0];
+#pragma unroll
+      for (int t = 1; t < n; ++t) {
+        const int m = ln.q0 + ln.qs * t;
+        const double uB = Uq[m], fB = Fq[m], wB = N[3 * Nq + m];
+        const double wv = max_nonneg_bits(wA, wB);
+        const double sum = dadd(fA, fB);
+        PH[ln.fs * t] = dfma(-(ln.visc ? signed_by(wv, ln.sg) : 0.0), dsub(uB, uA), q == 0 ? half(sum) : sum);
+        if (cfl && q == 0) base[Y::O_SW + ln.f0 + ln.fs * t] = wv;
+        uA = uB;
+        fA = fB;
+        wA = wB;
+      }
+      if (low_only) continue;
+      const double* F = base + Y::O_SF + q * C::NPH + lr * C::PPL;
+      double acc[n];
+#pragma unroll
+      for (int j = 0; j < n - 1; ++j) {
+        double s = 0.0;
+#pragma unroll
+        for (int i = n - 1; i > j; --i) {
+          s = ln.template suffix<TH>(i, j, F[i * (i - 1) / 2 + j], s);
+          acc[i] = j == 0 ? s : dadd(acc[i], s);
+        }
+      }
+#pragma unroll
+      for (int t = 1; t < n; ++t) DF[ln.fs * t] = dsub(acc[t], PH[ln.fs * t]);
+    }
+    __syncthreads();
   }
-  __syncthreads();
 
   // ---- node phase: low-order rhs (:139-243) and update, bounds' data, CFL
   double dt_loc = __longlong_as_double(0x7ff0000000000000LL);
@@ -558,7 +691,14 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
     double* R = base + Y::O_R + m;
     double* W = base + C::O_W + m;
     if (flags & F_CFL) {
-      const double lam = dfma(fabs(base[C::O_C + n + is]), R[Nq], dmul(fabs(base[C::O_C + ir]), R[0]));
+      double lx = R[0], ly = R[Nq];
+      if constexpr (SPLIT) {
+        const double* wx = base + Y::O_SW + (n + 1) * is + ir;
+        const double* wy = base + Y::O_SW + NSF + ir + n * is;
+        lx = dadd(wx[0], wx[1]);
+        ly = dadd(wy[0], wy[n]);
+      }
+      const double lam = dfma(fabs(base[C::O_C + n + is]), ly, dmul(fabs(base[C::O_C + ir]), lx));
       const double d = dmul(a.CFL * 0.5, rcp(lam));
       if (isnan(d)) nan_seen = true;
       dt_loc = fmin(dt_loc, d);
@@ -994,10 +1134,10 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
   }
 }
 
-template <int N1D, typename TH, bool EXT>
+template <int N1D, typename TH, bool EXT, bool SPLIT = false>
 __global__ void __launch_bounds__(FluxCfg<N1D>::THREADS) k_flux_a(StageArgs a) {
   extern __shared__ __align__(16) double sm[];
-  flux_a_body<N1D, TH, EXT>(a, blockIdx.x * a.epb, sm);
+  flux_a_body<N1D, TH, EXT, SPLIT>(a, blockIdx.x * a.epb, sm);
 }
 
 // =====================================================================================

@@ -21,12 +21,27 @@ struct StageGeometry {
   int elems_per_block_max_flux;
 };
 
-// Default threads per block of kernel A in flux form. Its longest phase, the lines, fills 64
-// threads at the default elements per block, and 128 leave half the block at that phase's
-// barrier (DMR 480x120 N=3: 776 us a stage with 128 threads, 656 with 64; KH 192x192 N=5:
-// 1659 and 1376). With few blocks per SM the shorter phases count, which 128 threads halve
-// (Riemann 64x64 N=4, 4.5 blocks an SM: 192 us with 128, 213 with 64).
-inline int flux_threads(int K, int epb) { return (K + epb - 1) / epb < 10 * 152 ? 128 : 64; }
+// Launch shape of kernel A in flux form: the layout of its lines (FluxLine: one thread a line,
+// or split), and the default elements and threads per block.
+//  * Split below 64k nodes (110k from N = 4 on, whose lines are longer): there an SM has so few
+//    warps that a line's chain is the stage's duration, and small blocks spread the elements
+//    evenly over the SMs. Measured, one thread a line against split, us a stage: KH 32x32 N=3
+//    37.4 and 26.9, 5x5 N=3 33.2 and 18.0, 16x16 N=2 26.7 and 17.0, 32x32 N=5 74.7 and 59.6,
+//    Riemann 64x64 N=4 with the intended bounds 206 and 157; KH 64x64 N=3 57.9 and 61.7, DMR
+//    480x120 N=3 611 and 645. The EXT modes (their time is in the bounds) keep the lines.
+//  * 64 threads otherwise: the lines fill them at the default elements per block, and 128 leave
+//    half the block at that phase's barrier (DMR 480x120 N=3 776 and 656 us, KH 192x192 N=5
+//    1659 and 1376); 128 where a grid is under ten blocks an SM and the shorter phases count.
+struct FluxShape {
+  bool split;
+  int epb, threads;
+};
+inline FluxShape flux_shape(int n1d, int K, int epb_lines, bool ext) {
+  const int64_t nodes = (int64_t)K * n1d * n1d;
+  if (!ext && nodes < (n1d >= 5 ? 110000 : 65536))
+    return {true, n1d == 2 ? 8 : n1d == 3 || n1d == 5 ? 3 : 2, 128};
+  return {false, epb_lines, (K + epb_lines - 1) / epb_lines < 10 * 152 ? 128 : 64};
+}
 
 template <int N1D>
 cudaError_t stage_prepare(StageGeometry* geo);

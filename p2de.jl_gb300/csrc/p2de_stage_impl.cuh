@@ -41,6 +41,12 @@ cudaError_t stage_prepare(StageGeometry* geo) {
   e = cudaFuncSetAttribute(k_flux_a<N1D, float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)F::template smem<true>(F::E_MAX));
   if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(k_flux_a<N1D, double, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)F::template smem<false, true>(F::E_SPLIT_MAX));
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(k_flux_a<N1D, float, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)F::template smem<false, true>(F::E_SPLIT_MAX));
+  if (e != cudaSuccess) return e;
   geo->elems_per_block_flux = F::E;
   geo->elems_per_block_max_flux = F::E_MAX;
   geo->elems_per_block = C::E;
@@ -62,6 +68,13 @@ cudaError_t launch_flux_a(const StageArgs& a, bool mixed, cudaStream_t st) {
   if (a.epb < 1 || a.epb > F::E_MAX || th % 32 != 0 || th > F::THREADS) return cudaErrorInvalidValue;
   const int grid = (a.K + a.epb - 1) / a.epb;
   const bool ext = a.flags & kExtFlags;
+  if (a.split && !ext && a.epb <= F::E_SPLIT_MAX) {
+    if (mixed)
+      k_flux_a<N1D, float, false, true><<<grid, th, F::template smem<false, true>(a.epb), st>>>(a);
+    else
+      k_flux_a<N1D, double, false, true><<<grid, th, F::template smem<false, true>(a.epb), st>>>(a);
+    return cudaGetLastError();
+  }
   if (mixed && ext)
     k_flux_a<N1D, float, true><<<grid, th, F::template smem<true>(a.epb), st>>>(a);
   else if (mixed)
