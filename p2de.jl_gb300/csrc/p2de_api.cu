@@ -700,7 +700,7 @@ int p2de_initialize_DG(const p2de_param* prm, const p2de_mesh* mesh, int device,
   a.CFL = prm->CFL;
   a.dt0 = prm->dt0;
   a.T = prm->T;
-  a.zeta = prm->zeta;
+  set_zeta(a, prm->zeta);
   a.ZEROTOL = prm->ZEROTOL;
   a.rhsL = s->rhsL;
   a.rhsH = s->rhsH;

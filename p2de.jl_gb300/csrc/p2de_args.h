@@ -100,7 +100,15 @@ struct StageArgs {
   // and FP32 gamma, gamma-1, 2 (gamma-1)
   double rgm1, hgm1, cws;
   float gasf[3];
+  // floor(log2((1 - zeta)/zeta)) (set_zeta): the quadratics' constant term is at least
+  // rho (zeta rhoe) 2^kzeta; very negative when zeta is not in (0, 1)
+  int kzeta;
 };
+
+inline void set_zeta(StageArgs& a, double zeta) {
+  a.zeta = zeta;
+  a.kzeta = zeta > 0.0 && zeta < 1.0 ? std::ilogb((1.0 - zeta) / zeta) : -100000;
+}
 
 inline void set_gas(StageArgs& a, double gamma) {
   a.gamma = gamma;

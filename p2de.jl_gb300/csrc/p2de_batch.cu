@@ -653,7 +653,7 @@ int p2de_batch_add(p2de_batch* b, const p2de_param* p, const p2de_mesh* m, const
   a.CFL = p->CFL;
   a.dt0 = p->dt0;
   a.T = p->T;
-  a.zeta = p->zeta;
+  set_zeta(a, p->zeta);
   a.ZEROTOL = p->ZEROTOL;
   a.rhsL = (double*)(base + lay.rhsL);
   a.rhsH = (double*)(base + lay.rhsH);

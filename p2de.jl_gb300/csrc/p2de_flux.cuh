@@ -47,22 +47,11 @@ __device__ __forceinline__ double half(double x) { return scale_exponent(x, -0x0
 __device__ __forceinline__ double twice(double x) { return scale_exponent(x, 0x00100000); }
 
 __device__ __forceinline__ bool negative(double x) { return __double2hiint(x) < 0; }
-// |x| > t (t > 0), x not NaN, by the bits
-__device__ __forceinline__ bool magnitude_above(double x, double t) {
-  const long long b = __double_as_longlong(x) & 0x7fffffffffffffffLL;
-  return b > __double_as_longlong(t) && b <= 0x7ff0000000000000LL;
-}
 // > 0 and not NaN, by the bits
 __device__ __forceinline__ bool positive_bits(double x) {
   const long long b = __double_as_longlong(x);
   return b > 0 && b <= 0x7ff0000000000000LL;
 }
-// max of two values that are >= 0 (or +NaN) by their bits
-__device__ __forceinline__ double max_nonneg_bits(double a, double b) {
-  const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
-  return __longlong_as_double(x > y ? x : y);
-}
-
 template <int N1D>
 struct FluxCfg {
   static constexpr int n = N1D;

@@ -219,7 +219,7 @@ extern "C" int p2de_rhs_noalloc(const p2de_param* prm, const p2de_device_mesh* m
   a.CFL = prm->CFL;
   a.dt0 = prm->dt0;
   a.T = prm->T;
-  a.zeta = prm->zeta;
+  set_zeta(a, prm->zeta);
   a.ZEROTOL = prm->ZEROTOL;
   double* data = scr + H_DATA;
   a.Lpre = data;

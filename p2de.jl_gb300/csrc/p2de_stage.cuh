@@ -86,7 +86,10 @@ struct Cfg {
   static constexpr size_t smem_a(int e) { return sizeof(double) * PER_ELEM_A * e + sizeof(int) * (NEV * e + 4); }
   static constexpr size_t SMEM_A = smem_a(E);
   // kernel B
-  static constexpr int PER_ELEM_B = 2 * NSF + 16 * NSF + 8 * NSF + 8;
+  static constexpr int O_FLIM = 2 * NSF;          // limited subcell fluxes [dir][face][c]
+  static constexpr int O_RJ = O_FLIM + 8 * NSF;   // 1/J
+  static constexpr int PER_ELEM_B = O_RJ + 2;
+  static_assert(O_FLIM % 2 == 0 && PER_ELEM_B % 2 == 0, "16-byte vectors");
   static constexpr size_t smem_b(int e) { return sizeof(double) * PER_ELEM_B * e; }
   static constexpr size_t SMEM_B = smem_b(E);
   // largest elements-per-block whose kernel-A shared memory fits 224 KB (capped at 32)
@@ -284,6 +287,18 @@ __device__ __forceinline__ double min_nonneg_bits(double a, double b) {
   return __longlong_as_double(x < y ? x : y);
 }
 
+// max of two values that are >= 0 (or +NaN) by their bits
+__device__ __forceinline__ double max_nonneg_bits(double a, double b) {
+  const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+  return __longlong_as_double(x > y ? x : y);
+}
+
+// |x| > t (t > 0), x not NaN, by the bits
+__device__ __forceinline__ bool magnitude_above(double x, double t) {
+  const long long b = __double_as_longlong(x) & 0x7fffffffffffffffLL;
+  return b > __double_as_longlong(t) && b <= 0x7ff0000000000000LL;
+}
+
 // fluxes(Dim2) (:175-194) with 1/rho given
 __device__ __forceinline__ void fluxes_r(const Gas<double>& g, const double* U, double rr, double* fx, double* fy) {
   double rho = U[0], rhou = U[1], rhov = U[2], E = U[3];
@@ -432,6 +447,35 @@ __device__ __forceinline__ double density_bound(double U0, double P0, double Lrh
     if (hi) l = fmin(l, fmax((Urho - U0) * rP, 0.0));
   }
   return l;
+}
+
+// Whether a node's factor for the flux difference fH - fL is exactly 1 under upper0 for P0 < 0,
+// decided on the integer pipe: with |fH_c - fL_c| bounded by the difference of their bits,
+// |P| < 2^X per component, U its low-order state and q = 4 dt / (wq J), the density bound is 1
+// when |P0| < U0/2, and a l^2 + b l + c of the internal-energy bound has no root in [0, 1] when
+// |a| + |b| < c/4 (|a| <= 2 2^2X, |b| <= 5 2^X max|U|, c >= rho (zeta rhoe) 2^kzeta, taken only
+// where c is well above the rounding of its terms). False when it is not settled so.
+__device__ __forceinline__ bool factor_is_one(const double* U, double Lrhoe, double q, const double* fH,
+                                              const double* fL, int kzeta) {
+  int X = -5000, S = -5000;
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    const long long h = __double_as_longlong(fH[c]), l = __double_as_longlong(fL[c]);
+    const int eh = (int)(h >> 52) & 0x7ff, el = (int)(l >> 52) & 0x7ff;
+    // both of one sign and exponent: |h - l| units of 2^(e - 1075); else each below 2^(e - 1022)
+    const long long d = h > l ? h - l : l - h;
+    const int x = ((h ^ l) >> 52) == 0 ? (el > 0 ? el : 1) - 1075 + 64 - __clzll(d) : (eh > el ? eh : el) - 1021;
+    X = x > X ? x : X;
+    const int u = ((int)(__double_as_longlong(U[c]) >> 52) & 0x7ff) - 1022;
+    S = u > S ? u : S;
+  }
+  const long long qb = __double_as_longlong(q), ub = __double_as_longlong(U[0]), lb = __double_as_longlong(Lrhoe);
+  if (qb < 0x0010000000000000LL || qb >= 0x7ff0000000000000LL || ub < 0x0010000000000000LL ||
+      lb < 0x0010000000000000LL)
+    return false;
+  X += (int)(qb >> 52) - 1022;
+  const int eu = (int)(ub >> 52) - 1023, c = eu + (int)(lb >> 52) - 1023 + kzeta;
+  return X < eu && c > 2 * S - 40 && X + S + 3 < c - 3 && 2 * X + 1 < c - 3;
 }
 
 // fS(::KPP{Dim2}) (KPP.jl:25-38), psi = (-cos u, sin u): the scalar fluxes in component 0
@@ -1093,29 +1137,29 @@ __device__ __forceinline__ void stage_a_body(const StageArgs& a, int k0, double*
       const double* G = base + C::O_GEO;
       int i = op.lp_i[pp], j = op.lp_j[pp], ax = op.lp_axis[pp];
       double S = op.lp_S[pp];
-      double g1 = ax == 0 ? G[1] : G[2], g2 = ax == 0 ? G[3] : G[4], gn = ax == 0 ? G[5] : G[8];
-      double S0x = g1 * S, S0y = g2 * S;
+      double gn = ax == 0 ? G[5] : G[8];
       double nn = fabs(S) * gn;
       double wsi = base[C::O_WS + 2 * i + ax], wsj = base[C::O_WS + 2 * j + ax];
-      double lam = nn * fmax(wsi, wsj);
+      double lam = nn * max_nonneg_bits(wsi, wsj);
       const double* Ui = base + C::O_U + 4 * i;
       const double* Uj = base + C::O_U + 4 * j;
       const double* Fi = base + C::O_FLUX + 8 * i;
       const double* Fj = base + C::O_FLUX + 8 * j;
       double* out = base + C::O_SCR + 9 * pp;
-      bool visc_x = fabs(S0x) > 1e-10;
       // 2 S0 * (fi + fj)/2 is S0 * (fi + fj) exactly (power-of-two factors)
       if (aa) {
         // the pair's terms on the other axis are zero; one instruction stream for both axes
         const int o = 4 * ax;
-        const double S0 = ax == 0 ? S0x : S0y;
-        const bool vis_on = ax == 0 ? visc_x : !visc_x;
+        const double S0 = (ax == 0 ? G[1] : G[4]) * S;
+        const bool vis_on = ax == 1 || magnitude_above(S0, 1e-10);
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           double vis = vis_on ? lam * (Uj[c] - Ui[c]) : 0.0;
           out[o + c] = fma(S0, Fi[o + c] + Fj[o + c], -vis);
         }
       } else {
+        const double S0x = (ax == 0 ? G[1] : G[2]) * S, S0y = (ax == 0 ? G[3] : G[4]) * S;
+        const bool visc_x = magnitude_above(S0x, 1e-10);
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           double vis = visc_x ? lam * (Uj[c] - Ui[c]) : 0.0;
@@ -1248,7 +1292,7 @@ __device__ __forceinline__ void stage_a_body(const StageArgs& a, int k0, double*
       double rrN = (code == BC_INTERIOR) ? rrP : rcp(Unb[0]);
       wsP = wavespeed_r(g, rrN, aa ? (xs ? Unb[1] : Unb[2]) : n1 * Unb[1] + n2 * Unb[2], Unb[3]);
     }
-    double lamB = 0.5 * nn * fmax(ws_own, wsP);
+    double lamB = 0.5 * nn * max_nonneg_bits(ws_own, wsP);
     double Fp[8];  // the projected face state's fluxes (projL)
     if (projL) fluxes_r(g, Uf, rcp(Uf[0]), Fp, Fp + 4);
     const double* Ff = projL ? Fp : base + C::O_FLUX + 8 * q;
@@ -1913,42 +1957,82 @@ __device__ __forceinline__ void stage_a_body(const StageArgs& a, int k0, double*
   // KPP evaluates no bound (subcell_bound_limiter!(dim, ::KPP), subcell.jl:389-402).
   if (!(flags & F_KPP)) {
   const bool upper0 = flags & F_REF_SEM;
-  for (int w = tid; w < Ke * NEV; w += bs) {
-    int e = w / NEV, r = w % NEV;
-    int dh = r / Nq, m = r % Nq;
-    int ir = m % n, is = m / n;
-    double* base = sm + e * PE;
-    const double* fb = base + C::O_SCR;
-    int d = dh >> 1, h = dh & 1;
-    int fi = (d == 0) ? (ir + h) + (n + 1) * is : ir + n * (is + h);
-    const double* fH = fb + ((d * 2 + 0) * NSF + fi) * 4;
-    const double* fL = fb + ((d * 2 + 1) * NSF + fi) * 4;
-    const double* uL = base + C::O_PRIM + 6 * m;
-    double P0 = (fH[0] - fL[0]) * uL[5];
-    if (h == 0) P0 = -P0;
-    const double* lim = base + C::O_RHSL + 4 * m;
-    base[C::O_EV + r] = density_bound(uL[0], P0, lim[0], upper0 ? 0.0 : lim[2], upper0, lim[1]);
-  }
-  __syncthreads();
-  for (int w = tid; w < Ke * NEV; w += bs) {
-    int e = w / NEV, r = w % NEV;
-    int dh = r / Nq, m = r % Nq;
-    int ir = m % n, is = m / n;
-    const double* ev = sm + e * PE + C::O_EV;
-    if (is_zero_bits(ev[r])) continue;
-    int d = dh >> 1, h = dh & 1;
-    // the other evaluation of the same face, if the face is interior
-    int partner = -1;
-    if (d == 0) {
-      if (h == 0 && ir > 0) partner = 1 * Nq + (ir - 1) + n * is;
-      if (h == 1 && ir + 1 < n) partner = 0 * Nq + (ir + 1) + n * is;
+  // One item per face, the interior faces of all elements first. Under upper0 a node with
+  // U0 >= Lrho > 0 and P0 >= +0 has factor 0 (density_bound), and the sign of P0 is that of
+  // fH0 - fL0: of the two nodes of an interior face one always has it, so the face is settled
+  // by integer comparisons of fH0 and fL0. A boundary face with fH = fL has P = -0 at its upper
+  // node: factor 1, no solve; one whose difference is rounding is settled by factor_is_one.
+  constexpr int NI = 2 * n * (n - 1);
+  for (int w = tid; w < Ke * 2 * NSF; w += bs) {
+    const int e = w < Ke * NI ? w / NI : (w - Ke * NI) / (4 * n);
+    const int r = w < Ke * NI ? w % NI : NI + (w - Ke * NI) % (4 * n);
+    int d, t, l;  // direction, face position on the line, line
+    if (r < NI) {
+      d = r / (NI / 2);
+      const int q = r % (NI / 2);
+      t = d == 0 ? q % (n - 1) + 1 : q / n + 1;
+      l = d == 0 ? q / (n - 1) : q % n;
     } else {
-      if (h == 0 && is > 0) partner = 3 * Nq + ir + n * (is - 1);
-      if (h == 1 && is + 1 < n) partner = 2 * Nq + ir + n * (is + 1);
+      const int q = r - NI;
+      d = q / (2 * n);
+      t = (q / n) % 2 ? n : 0;
+      l = q % n;
     }
-    if (partner >= 0 && is_zero_bits(ev[partner])) continue;
-    int slot = atomicAdd(&s_list[0], 1);
-    s_list[1 + slot] = e * NEV + r;
+    double* base = sm + e * PE;
+    double* ev = base + C::O_EV;
+    const int fi = d == 0 ? t + (n + 1) * l : l + n * t;
+    const double* fH = base + C::O_SCR + ((d * 2 + 0) * NSF + fi) * 4;
+    const double* fL = base + C::O_SCR + ((d * 2 + 1) * NSF + fi) * 4;
+    const long long hb = __double_as_longlong(fH[0]), lb = __double_as_longlong(fL[0]);
+    const bool finite = (hb & 0x7ff0000000000000LL) != 0x7ff0000000000000LL &&
+                        (lb & 0x7ff0000000000000LL) != 0x7ff0000000000000LL;
+    const bool up = order_key(fH[0]) >= order_key(fL[0]);  // fH0 - fL0 is not negative
+    // node on side h of the face: 0 the node above it (whose lower face it is), 1 below it
+    auto node = [&](int h) {
+      const int i = h ? t - 1 : t;
+      return i < 0 || i >= n ? -1 : d == 0 ? i + n * l : l + n * i;
+    };
+    bool zero = false, solve[2] = {false, false};
+    double f[2] = {1.0, 1.0};
+    bool ok[2] = {false, false};
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int m = node(h);
+      if (m < 0 || !upper0 || !finite) continue;
+      const double* uL = base + C::O_PRIM + 6 * m;
+      const long long U0 = __double_as_longlong(uL[0]), Lr = __double_as_longlong(base[C::O_RHSL + 4 * m]),
+                      q = __double_as_longlong(uL[5]);
+      ok[h] = U0 > 0 && U0 < 0x7ff0000000000000LL && Lr <= U0 && q > 0 && q < 0x7ff0000000000000LL;
+      if (ok[h] && (h == 1) == up) zero = true;
+    }
+    if (!zero) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int m = node(h);
+        if (m < 0) continue;
+        const double* uL = base + C::O_PRIM + 6 * m;
+        const double* lim = base + C::O_RHSL + 4 * m;
+        if (ok[h]) {
+          bool same = true;
+#pragma unroll
+          for (int c = 0; c < 4; ++c) same = same && __double_as_longlong(fH[c]) == __double_as_longlong(fL[c]);
+          if (same || (!(flags & F_TVD) && factor_is_one(uL, uL[4], uL[5], fH, fL, a.kzeta))) continue;
+        }
+        double P0 = (fH[0] - fL[0]) * uL[5];
+        if (h == 0) P0 = -P0;
+        f[h] = density_bound(uL[0], P0, lim[0], upper0 ? 0.0 : lim[2], upper0, lim[1]);
+        solve[h] = true;
+      }
+      zero = is_zero_bits(f[0]) || is_zero_bits(f[1]);
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int m = node(h);
+      if (m < 0) continue;
+      const int q = (2 * d + h) * Nq + m;
+      ev[q] = zero ? 0.0 : f[h];
+      if (!zero && solve[h]) s_list[1 + atomicAdd(&s_list[0], 1)] = e * NEV + q;
+    }
   }
   __syncthreads();
   const int nlist = s_list[0];
@@ -2256,16 +2340,12 @@ __device__ __forceinline__ void stage_b_body(const StageArgs& a, int k0, double*
   else
     dt = a.scal[S_DT];
   const bool limited = flags & F_DO_LIMIT;
-  // smem: L [2 NSF], fbar [16 NSF], flim [8 NSF], 1/J
+  // smem: L [2 NSF], flim [8 NSF], 1/J
   if (limited) {
-    for (int e = tid; e < Ke; e += bs) sm[e * PE + 26 * NSF] = rcp(a.geom[5 * (size_t)(k0 + e)]);
+    for (int e = tid; e < Ke; e += bs) sm[e * PE + C::O_RJ] = rcp(a.geom[5 * (size_t)(k0 + e)]);
     for (int w = tid; w < Ke * 2 * NSF; w += bs) {
       int e = w / (2 * NSF), r = w % (2 * NSF);
       sm[e * PE + r] = a.Lpre[(size_t)(k0 + e) * 2 * NSF + r];
-    }
-    for (int w = tid; w < Ke * C::FBAR; w += bs) {
-      int e = w / C::FBAR, r = w % C::FBAR;
-      sm[e * PE + 2 * NSF + r] = a.fbar[(size_t)(k0 + e) * C::FBAR + r];
     }
     __syncthreads();
     // symmetrize_limiting_parameters!(::Dim2) with subcell_index_P_x/y (limiter_utils.jl:179-237)
@@ -2298,17 +2378,41 @@ __device__ __forceinline__ void stage_b_body(const StageArgs& a, int k0, double*
       sm[e * PE + d * NSF + idx] = fmin(own, par);
     }
     __syncthreads();
-    // accumulate_f_bar_limited!(::Dim2) (subcell.jl:841-876)
-    for (int w = tid; w < Ke * 2 * NSF * 4; w += bs) {
-      int e = w / (2 * NSF * 4), r = w % (2 * NSF * 4);
-      int d = r / (NSF * 4), fi = (r / 4) % NSF, c = r % 4;
+    // accumulate_f_bar_limited!(::Dim2) (subcell.jl:841-876), one face per thread, the interior
+    // faces of all elements first: a face with factor 0 (under the reference's reading, every
+    // interior one) takes fL without reading fH and without an FP64 instruction
+    constexpr int NI = 2 * n * (n - 1);
+    for (int w = tid; w < Ke * 2 * NSF; w += bs) {
+      const int e = w < Ke * NI ? w / NI : (w - Ke * NI) / (4 * n);
+      const int r = w < Ke * NI ? w % NI : NI + (w - Ke * NI) % (4 * n);
+      int d, t, ln;
+      if (r < NI) {
+        d = r / (NI / 2);
+        const int q = r % (NI / 2);
+        t = d == 0 ? q % (n - 1) + 1 : q / n + 1;
+        ln = d == 0 ? q / (n - 1) : q % n;
+      } else {
+        const int q = r - NI;
+        d = q / (2 * n);
+        t = (q / n) % 2 ? n : 0;
+        ln = q % n;
+      }
+      const int fi = d == 0 ? t + (n + 1) * ln : ln + n * t;
       double* base = sm + e * PE;
-      double l = base[d * NSF + fi];
-      const double* fb = base + 2 * NSF;
-      double fH = fb[((d * 2 + 0) * NSF + fi) * 4 + c];
-      double fL = fb[((d * 2 + 1) * NSF + fi) * 4 + c];
+      const double l = base[d * NSF + fi];
+      const double2* g = reinterpret_cast<const double2*>(a.fbar + (size_t)(k0 + e) * C::FBAR + (d * 2 * NSF + fi) * 4);
+      double2 lo = g[2 * NSF], hi = g[2 * NSF + 1];
       // l fH + (1 - l) fL as fL + l (fH - fL): one rounding fewer, and exactly fL at l = 0
-      base[2 * NSF + 16 * NSF + (d * NSF + fi) * 4 + c] = fma(l, fH - fL, fL);
+      if (!is_zero_bits(l)) {
+        const double2 h0 = g[0], h1 = g[1];
+        lo.x = fma(l, h0.x - lo.x, lo.x);
+        lo.y = fma(l, h0.y - lo.y, lo.y);
+        hi.x = fma(l, h1.x - hi.x, hi.x);
+        hi.y = fma(l, h1.y - hi.y, hi.y);
+      }
+      double2* out = reinterpret_cast<double2*>(base + C::O_FLIM + (d * NSF + fi) * 4);
+      out[0] = lo;
+      out[1] = hi;
     }
     __syncthreads();
   }
@@ -2322,8 +2426,8 @@ __device__ __forceinline__ void stage_b_body(const StageArgs& a, int k0, double*
     double ru[4];
     size_t gidx = ((size_t)k * Nq + m) * 4;
     if (limited) {
-      const double* fl = sm + e * PE + 2 * NSF + 16 * NSF;
-      double rwJ = sm[e * PE + 26 * NSF] * op.rwq[m];  // (1/J)(1/wq)
+      const double* fl = sm + e * PE + C::O_FLIM;
+      double rwJ = sm[e * PE + C::O_RJ] * op.rwq[m];  // (1/J)(1/wq)
       const double* fx0 = fl + ((0 * NSF) + ir + (n + 1) * is) * 4;
       const double* fx1 = fl + ((0 * NSF) + ir + 1 + (n + 1) * is) * 4;
       const double* fy0 = fl + ((1 * NSF) + ir + n * is) * 4;
