@@ -203,10 +203,11 @@ __device__ __forceinline__ double rhoe_root(const double* U, const double* dF, d
 }
 
 // phi = rhoe rho^-gamma (s_modified_ufun) of U + l P, explicitly rounded
-__device__ __forceinline__ double phi_at(const double* U, const double* P, double l, double gamma) {
+__device__ __forceinline__ double phi_at(const double* U, const double* P, double l, double gamma,
+                                         const OpTable& op) {
   const double r = dfma(l, P[0], U[0]), m1 = dfma(l, P[1], U[1]), m2 = dfma(l, P[2], U[2]), E = dfma(l, P[3], U[3]);
   const double rhoe = dfma(-0.5, dmul(dfma(m1, m1, dmul(m2, m2)), rcp(r)), E);
-  return dmul(rhoe, pow(r, -gamma));
+  return dmul(rhoe, pow_fast(r, -gamma, op));
 }
 
 // Along-axis values of one line node: the state (rho, normal and tangential momentum, E) and
@@ -740,9 +741,9 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
       // node and its stencil) + (1 - eps_k) phi_min; eps_k = 1 unless relaxed
       const double z[4] = {0.0, 0.0, 0.0, 0.0};
       const double Uo[4] = {U[0], U[Nq], U[2 * Nq], U[3 * Nq]};
-      double lb = phi_at(Uo, z, 0.0, a.gamma);
+      double lb = phi_at(Uo, z, 0.0, a.gamma, op);
 #pragma unroll 1
-      for (int t = 0; t < 4; ++t) lb = fmin(lb, phi_at(a.Uq + 4 * stencil(t), z, 0.0, a.gamma));
+      for (int t = 0; t < 4; ++t) lb = fmin(lb, phi_at(a.Uq + 4 * stencil(t), z, 0.0, a.gamma, op));
       if (flags & F_RELAXED) {
         const double eps = base[Y::O_X];
         lb = dfma(eps, lb, dmul(dsub(1.0, eps), a.phimin[0]));
@@ -895,7 +896,7 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
         const double P[4] = {dmul(s, dF[0]), dmul(s, dF[1]), dmul(s, dF[2]), dmul(s, dF[3])};
         const double lden = density_bound(uL[0], P[0], W[C::W_LRHO * Nq], W[C::W_URHO * Nq], false, 0.0);
         lm = fmin(fmin(lden, lm), 1.0);
-        if (!(phi_at(uL, P, lm, a.gamma) >= W[C::W_THR * Nq])) {
+        if (!(phi_at(uL, P, lm, a.gamma, op) >= W[C::W_THR * Nq])) {
           const int id = 2 * s_list[w] + h;
           base[C::O_W + (C::W_EV + 2 * d + h) * Nq + m] = lm;
           s_bis[atomicAdd(&s_cnt[1], 1)] = id;
@@ -928,7 +929,7 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
       double good = 0.0, bad = *ev;
       for (int it = 0; it <= 20; ++it) {
         const double mid = dmul(0.5, dadd(good, bad));
-        if (phi_at(uL, P, mid, a.gamma) >= thr)
+        if (phi_at(uL, P, mid, a.gamma, op) >= thr)
           good = mid;
         else
           bad = mid;

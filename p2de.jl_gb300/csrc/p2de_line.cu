@@ -21,6 +21,7 @@
 #include <cstring>
 
 #include "p2de_args.h"
+#include "p2de_arith.cuh"
 #include "p2de_line.h"
 #include "p2de_physics.cuh"
 
@@ -86,49 +87,51 @@ __device__ __forceinline__ bool done(const LineArgs& a) { return a.ts[TS_DONE] !
 
 // ---- point functions (compressible_Navier_Stokes.jl; four slots, y momentum 0) ----------
 __device__ double pfun4(double gamma, const double* U) {
-  return (gamma - 1.0) * (U[3] - 0.5 * (U[1] * U[1] + U[2] * U[2]) / U[0]);
+  return (gamma - 1.0) * (U[3] - div_rn(0.5 * (U[1] * U[1]), U[0]));
 }
-__device__ double rhoe4(const double* U) { return U[3] - 0.5 * (U[1] * U[1] + U[2] * U[2]) / U[0]; }
-__device__ double betafun4(double gamma, const double* U) { return U[0] / (2.0 * pfun4(gamma, U)); }
+__device__ double rhoe4(const double* U) { return U[3] - div_rn(0.5 * (U[1] * U[1]), U[0]); }
+__device__ double betafun4(double gamma, const double* U) { return div_rn(U[0], 2.0 * pfun4(gamma, U)); }
 // wavespeed_estimate(::Dim1) (:48-52) of (rho, un, E)
 __device__ double wavespeed1(double gamma, double rho, double rhou, double E) {
-  const double p = (gamma - 1.0) * (E - 0.5 * (rhou * rhou) / rho);
-  return fabs(rhou / rho) + sqrt(gamma * p / rho);
+  const double p = (gamma - 1.0) * (E - div_rn(0.5 * (rhou * rhou), rho));
+  return fabs(div_rn(rhou, rho)) + sqrt_rn(div_rn(gamma * p, rho));
 }
 __device__ double wavespeed4(double gamma, const double* U, double n1, double n2) {
   return wavespeed1(gamma, U[0], n1 * U[1] + n2 * U[2], U[3]);
 }
 __device__ void fluxes4(double gamma, const double* U, double* f) {  // the x flux
-  const double rho = U[0], rhou = U[1], rhov = U[2], E = U[3];
+  const double rho = U[0], rhou = U[1], E = U[3];
   const double p = pfun4(gamma, U);
-  const double u = rhou / rho, v = rhov / rho;
+  const double u = div_rn(rhou, rho);
   f[0] = rhou;
   f[1] = rhou * u + p;
-  f[2] = rho * u * v;
+  f[2] = 0.0;
   f[3] = u * (E + p);
 }
-__device__ void v_ufun4(double gamma, const double* U, double* V) {
+__device__ void v_ufun4(const LineOps& o, double gamma, const double* U, double* V) {
   const double p = pfun4(gamma, U);
-  const double s = log(p / pow(U[0], gamma));
-  V[0] = (gamma + 1.0 - s) - (gamma - 1.0) * U[3] / p;
-  V[1] = U[1] * (gamma - 1.0) / p;
-  V[2] = U[2] * (gamma - 1.0) / p;
-  V[3] = -U[0] * (gamma - 1.0) / p;
+  const double s = log_fast(div_rn(p, pow_fast(U[0], gamma, o)), o);
+  V[0] = (gamma + 1.0 - s) - div_rn((gamma - 1.0) * U[3], p);
+  V[1] = div_rn(U[1] * (gamma - 1.0), p);
+  V[2] = 0.0;
+  V[3] = div_rn(-U[0] * (gamma - 1.0), p);
 }
-__device__ void u_vfun4(double gamma, const double* V, double* U) {
-  const double s = gamma - V[0] + (V[1] * V[1] + V[2] * V[2]) / (2.0 * V[3]);
-  const double rhoeV = pow((gamma - 1.0) / pow(-V[3], gamma), 1.0 / (gamma - 1.0)) * exp(-s / (gamma - 1.0));
+__device__ void u_vfun4(const LineOps& o, double gamma, const double* V, double* U) {
+  const double q = div_rn(V[1] * V[1], 2.0 * V[3]);
+  const double s = gamma - V[0] + q;
+  const double rhoeV = pow_fast(div_rn(gamma - 1.0, pow_fast(-V[3], gamma, o)), div_rn(1.0, gamma - 1.0), o) *
+                       exp_fast(div_rn(-s, gamma - 1.0), o);
   U[0] = -rhoeV * V[3];
   U[1] = rhoeV * V[1];
-  U[2] = rhoeV * V[2];
-  U[3] = rhoeV * (1.0 - (V[1] * V[1] + V[2] * V[2]) / (2.0 * V[3]));
+  U[2] = 0.0;
+  U[3] = rhoeV * (1.0 - q);
 }
 // logmean (:307-321)
 __device__ double logmean(double aL, double aR, double logL, double logR) {
   const double da = aR - aL, aavg = 0.5 * (aR + aL);
-  const double f = da / aavg, v = f * f;
+  const double f = div_rn(da, aavg), v = f * f;
   if (fabs(f) < 1e-4) return aavg * (1.0 + v * (-0.2 - v * (0.0512 - v * 0.026038857142857)));
-  return -da / (logL - logR);
+  return div_rn(-da, logL - logR);
 }
 // fS (:196-218) as the Dim2 x flux with v = 0; U = (rho, u, v, beta, log rho, log beta)
 __device__ void fS4(double gamma, const double* UL, const double* UR, double* F) {
@@ -136,17 +139,16 @@ __device__ void fS4(double gamma, const double* UL, const double* UR, double* F)
   const double betalog = logmean(UL[3], UR[3], UL[5], UR[5]);
   const double rhoavg = 0.5 * (UL[0] + UR[0]);
   const double uavg = 0.5 * (UL[1] + UR[1]);
-  const double vavg = 0.5 * (UL[2] + UR[2]);
-  const double unorm = UL[1] * UR[1] + UL[2] * UR[2];
-  const double pa = rhoavg / (UL[3] + UR[3]);
-  const double f4aux = rholog / (2.0 * (gamma - 1.0) * betalog) + pa + 0.5 * rholog * unorm;
+  const double unorm = UL[1] * UR[1];
+  const double pa = div_rn(rhoavg, UL[3] + UR[3]);
+  const double f4aux = div_rn(rholog, 2.0 * (gamma - 1.0) * betalog) + pa + 0.5 * rholog * unorm;
   const double FxS1 = rholog * uavg;
   F[0] = FxS1;
   F[1] = FxS1 * uavg + pa;
-  F[2] = FxS1 * vavg;
+  F[2] = 0.0;
   F[3] = f4aux * uavg;
 }
-__device__ double s_modified4(double gamma, const double* U) { return rhoe4(U) * pow(U[0], -gamma); }
+__device__ double s_modified4(const LineOps& o, double gamma, const double* U) { return rhoe4(U) * pow_fast(U[0], -gamma, o); }
 // isless on Float64 (NaN last, -0.0 before 0.0)
 __device__ bool jisless(double a, double b) {
   if (isnan(a)) return false;
@@ -170,8 +172,9 @@ __device__ double rhoe_quadratic_solve(const double* U, const double* P, double 
   const double c = U[3] * U[0] - 1.0 / 2.0 * (U[1] * U[1] + U[2] * U[2]) - U[0] * Lrhoe;
   double l = 1.0;
   if (b * b - 4.0 * a * c >= 0.0) {
-    const double r1 = (-b + sqrt(b * b - 4.0 * a * c)) / (2.0 * a);
-    const double r2 = (-b - sqrt(b * b - 4.0 * a * c)) / (2.0 * a);
+    const double sq = sqrt_rn(b * b - 4.0 * a * c);
+    const double r1 = div_rn(-b + sq, 2.0 * a);
+    const double r2 = div_rn(-b - sq, 2.0 * a);
     if (r1 > ZEROTOL && r2 > ZEROTOL)
       l = jmin(r1, r2);
     else if (r1 > ZEROTOL && r2 < -ZEROTOL)
@@ -185,8 +188,8 @@ __device__ double rhoe_quadratic_solve(const double* U, const double* P, double 
 __device__ double bound_rho_rhoe(const double* U, const double* P, double Lrho, double Lrhoe, double Urho,
                                  double Urhoe, double ZEROTOL) {
   double l = 1.0;
-  if (U[0] + P[0] < Lrho) l = jmax((Lrho - U[0]) / P[0], 0.0);
-  if (U[0] + P[0] > Urho) l = jmin(l, jmax((Urho - U[0]) / P[0], 0.0));
+  if (U[0] + P[0] < Lrho) l = jmax(div_rn(Lrho - U[0], P[0]), 0.0);
+  if (U[0] + P[0] > Urho) l = jmin(l, jmax(div_rn(Urho - U[0], P[0]), 0.0));
   return jmin(jmin(l, rhoe_quadratic_solve(U, P, Lrhoe, ZEROTOL)), rhoe_quadratic_solve(U, P, Urhoe, ZEROTOL));
 }
 // find_alpha (low_order_graph_viscosity.jl:316-345), the doubling bounded
@@ -235,7 +238,7 @@ __device__ void Bx(const LineArgs& a, int k, int f, double& b0, double& b1) {
 __device__ double norm2(double x, double y) {
   const double m = fmax(fabs(x), fabs(y));
   if (m == 0.0 || isinf(m) || isnan(m)) return m;
-  return sqrt(x * x + y * y);
+  return sqrt_rn(x * x + y * y);
 }
 
 // smoothness indicator (shock_capture.jl:14-45), blending factor (:118-137) and smoothness
@@ -329,7 +332,7 @@ __global__ void k_line_face(LineArgs a) {
   double U[MQ][4], v[MQ][4];
   for (int i = 0; i < n; ++i) {
     ld4(a.Uq + 4 * ((size_t)n * k + i), U[i]);
-    v_ufun4(a.gamma, U[i], v[i]);
+    v_ufun4(*a.ops, a.gamma, U[i], v[i]);
   }
   {
     const int fn = f == 0 ? 0 : N;
@@ -353,7 +356,7 @@ __global__ void k_line_face(LineArgs a) {
         double vt[4], ut[4];
         face_var(t, vt);
         if (!(vt[3] < -eps)) return false;
-        u_vfun4(a.gamma, vt, ut);
+        u_vfun4(*a.ops, a.gamma, vt, ut);
         const double rho = ut[0], re = rhoe4(ut);
         return vt[3] < jmin(zeta * VUf[3], -eps) && rho > jmax((1 - eta) * Ufv[0], eps) && rho < (1 + eta) * Ufv[0] &&
                re > jmax((1 - eta) * rhoef, eps) && re < (1 + eta) * rhoef;
@@ -375,7 +378,7 @@ __global__ void k_line_face(LineArgs a) {
     a.theta[2 * ((size_t)a.K * s + k) + f] = th;
     double acc[4], u[4];
     face_var(th, acc);
-    u_vfun4(a.gamma, acc, u);
+    u_vfun4(*a.ops, a.gamma, acc, u);
     st4(a.uf + 4 * (2 * (size_t)k + f), u);
   }
 }
@@ -404,7 +407,7 @@ __global__ void k_line_face_team(LineArgs a) {
   __shared__ double sU[n][4], sv[n][4];
   if (threadIdx.x < n) {
     ld4(a.Uq + 4 * ((size_t)n * k + threadIdx.x), sU[threadIdx.x]);
-    v_ufun4(a.gamma, sU[threadIdx.x], sv[threadIdx.x]);
+    v_ufun4(*a.ops, a.gamma, sU[threadIdx.x], sv[threadIdx.x]);
   }
   __syncthreads();
   const int fn = f == 0 ? 0 : N;
@@ -431,7 +434,7 @@ __global__ void k_line_face_team(LineArgs a) {
       double vt[4];
       face_var(t, vt);
       if (!(vt[3] < -eps)) return false;
-      u_vfun4(a.gamma, vt, ut);
+      u_vfun4(*a.ops, a.gamma, vt, ut);
       const double rho = ut[0], re = rhoe4(ut);
       return vt[3] < jmin(zeta * VUf[3], -eps) && rho > jmax((1 - eta) * Ufv[0], eps) && rho < (1 + eta) * Ufv[0] &&
              re > jmax((1 - eta) * rhoef, eps) && re < (1 + eta) * rhoef;
@@ -494,7 +497,7 @@ __global__ void k_line_face_team(LineArgs a) {
     if (!have_u) {
       double acc[4];
       face_var(th, acc);
-      u_vfun4(a.gamma, acc, u);
+      u_vfun4(*a.ops, a.gamma, acc, u);
     }
     st4(a.uf + 4 * (2 * (size_t)k + f), u);
   }
@@ -522,7 +525,7 @@ __global__ void k_line_low(LineArgs a) {
     const int i = j + 1;
     const double Sr0 = 0.5 * (-0.5 - 0.5), Ss0 = 0.0;
     const double S0 = g[1] * Sr0 + g[2] * Ss0, S1 = g[3] * Sr0 + g[4] * Ss0;
-    const double nn = norm2(S0, S1), n1 = S0 / nn, n2 = S1 / nn;
+    const double nn = norm2(S0, S1), n1 = div_rn(S0, nn), n2 = div_rn(S1, nn);
     const double ws = jmax(wavespeed4(a.gamma, U[i], n1, n2), wavespeed4(a.gamma, U[j], -n1, -n2));
     const double lij = nn * ws;
     lamR[j] = lij;
@@ -546,8 +549,8 @@ __global__ void k_line_low(LineArgs a) {
     Bx(a, k, f, b0, b1);
     Bx(a, kP, iP, bP0, bP1);
     const double nn = norm2(b0, b1), nnP = norm2(bP0, bP1);
-    wsf[f] = wavespeed4(a.gamma, Uf, b0 / nn, b1 / nn);
-    const double wsP = wavespeed4(a.gamma, UfP, bP0 / nnP, bP1 / nnP);
+    wsf[f] = wavespeed4(a.gamma, Uf, div_rn(b0, nn), div_rn(b1, nn));
+    const double wsP = wavespeed4(a.gamma, UfP, div_rn(bP0, nnP), div_rn(bP1, nnP));
     const int8_t bc = a.bc[fk];
     if (bc == BC_INFLOW) {
       const double* I = a.Ival + 3 * (size_t)a.bcidx[fk];
@@ -574,7 +577,7 @@ __global__ void k_line_low(LineArgs a) {
   for (int i = 0; i < n; ++i) {
     const double wJq = J * o.wq[i];
     double rl[4];
-    for (int c = 0; c < 4; ++c) rl[c] = r[i][c] / wJq + 0.0;
+    for (int c = 0; c < 4; ++c) rl[c] = div_rn(r[i][c], wJq) + 0.0;
     st4(a.rhsL + 4 * ((size_t)n * k + i), rl);
     if (a.flags & LF_RHSU_L) st4(a.rhsU + 4 * ((size_t)n * k + i), rl);
   }
@@ -595,7 +598,7 @@ __global__ void k_line_low(LineArgs a) {
         }
       }
       const double wJq = J * o.wq[i];
-      dtl = jmin(dtl, a.CFL * 0.5 * wJq / li);
+      dtl = jmin(dtl, div_rn(a.CFL * 0.5 * wJq, li));
     }
     if (dtl > 0.0)
       atomicMin(&a.dtkey[0], (unsigned long long)__double_as_longlong(dtl));
@@ -639,7 +642,7 @@ __global__ void k_line_low_team(LineArgs a) {
     const int j = lane, i = j + 1;
     const double Sr0 = 0.5 * (-0.5 - 0.5), Ss0 = 0.0;
     const double S0 = g[1] * Sr0 + g[2] * Ss0, S1 = g[3] * Sr0 + g[4] * Ss0;
-    const double nn = norm2(S0, S1), n1 = S0 / nn, n2 = S1 / nn;
+    const double nn = norm2(S0, S1), n1 = div_rn(S0, nn), n2 = div_rn(S1, nn);
     const double ws = jmax(wavespeed4(a.gamma, U[i], n1, n2), wavespeed4(a.gamma, U[j], -n1, -n2));
     const double lij = nn * ws;
     lamR[j] = lij;
@@ -659,8 +662,8 @@ __global__ void k_line_low_team(LineArgs a) {
     Bx(a, k, f, b0, b1);
     Bx(a, kP, iP, bP0, bP1);
     const double nn = norm2(b0, b1), nnP = norm2(bP0, bP1);
-    wsf[f] = wavespeed4(a.gamma, Uf, b0 / nn, b1 / nn);
-    const double wsP = wavespeed4(a.gamma, UfP, bP0 / nnP, bP1 / nnP);
+    wsf[f] = wavespeed4(a.gamma, Uf, div_rn(b0, nn), div_rn(b1, nn));
+    const double wsP = wavespeed4(a.gamma, UfP, div_rn(bP0, nnP), div_rn(bP1, nnP));
     const int8_t bc = a.bc[fk];
     if (bc == BC_INFLOW) {
       const double* I = a.Ival + 3 * (size_t)a.bcidx[fk];
@@ -697,7 +700,7 @@ __global__ void k_line_low_team(LineArgs a) {
       for (int c = 0; c < 4; ++c) r[c] = r[c] - BF[1][c];
     const double wJq = J * o.wq[m];
     double rl[4];
-    for (int c = 0; c < 4; ++c) rl[c] = r[c] / wJq + 0.0;
+    for (int c = 0; c < 4; ++c) rl[c] = div_rn(r[c], wJq) + 0.0;
     st4(a.rhsL + 4 * ((size_t)n * k + m), rl);
     if (a.flags & LF_RHSU_L) st4(a.rhsU + 4 * ((size_t)n * k + m), rl);
     if (a.flags & LF_CFL) {
@@ -715,7 +718,7 @@ __global__ void k_line_low_team(LineArgs a) {
           li += lamB[f];
         }
       }
-      scand[e][i] = a.CFL * 0.5 * wJq / li;
+      scand[e][i] = div_rn(a.CFL * 0.5 * wJq, li);
     }
   }
   if (!(a.flags & LF_CFL)) return;
@@ -736,7 +739,7 @@ __global__ void k_line_phimin(LineArgs a) {
   if (g >= (long long)a.K * a.N1D || done(a) || a.ts[TS_PHI] == 0.0) return;
   double U[4];
   ld4(a.Uq + 4 * g, U);
-  atomicMin(a.phikey, encode_key(s_modified4(a.gamma, U)));
+  atomicMin(a.phikey, encode_key(s_modified4(*a.ops, a.gamma, U)));
 }
 
 // the volume two-point terms S_ij fS(u_i, u_j) of flux_differencing_volume!
@@ -759,8 +762,8 @@ __global__ void k_line_pairs(LineArgs a) {
   state(i, ui);
   state(j, uj);
   const double bi = betafun4(a.gamma, ui), bj = betafun4(a.gamma, uj);
-  const double Ui[6] = {ui[0], ui[1] / ui[0], ui[2] / ui[0], bi, log(ui[0]), log(bi)};
-  const double Uj[6] = {uj[0], uj[1] / uj[0], uj[2] / uj[0], bj, log(uj[0]), log(bj)};
+  const double Ui[6] = {ui[0], div_rn(ui[1], ui[0]), 0.0, bi, log_fast(ui[0], o), log_fast(bi, o)};
+  const double Uj[6] = {uj[0], div_rn(uj[1], uj[0]), 0.0, bj, log_fast(uj[0], o), log_fast(bj, o)};
   const double* gg = a.geom + 5 * (size_t)k;
   const double Sr = o.Sh[i + Nh * j], Ss = 0.0;
   const double S0 = gg[1] * Sr + gg[2] * Ss;
@@ -803,8 +806,8 @@ __global__ void k_line_high(LineArgs a) {
     Bx(a, k, f, b0, b1);
     Bx(a, kP, iP, c0, c1);
     const double nn = norm2(b0, b1), nnP = norm2(c0, c1);
-    const double lam = wavespeed4(a.gamma, ut[n + f], b0 / nn, b1 / nn);
-    const double lamP = wavespeed4(a.gamma, uP[f], c0 / nnP, c1 / nnP);
+    const double lam = wavespeed4(a.gamma, ut[n + f], div_rn(b0, nn), div_rn(b1, nn));
+    const double lamP = wavespeed4(a.gamma, uP[f], div_rn(c0, nnP), div_rn(c1, nnP));
     LFc[f] = 0.5 * nn * jmax(lam, lamP);
     const int8_t bc = a.bc[fk];
     if (bc == BC_INFLOW || bc == BC_OUTFLOW) {
@@ -847,7 +850,7 @@ __global__ void k_line_high(LineArgs a) {
   const bool limited = th0 < 1.0 || th1 < 1.0;
   double rH[MQ][4], rL[MQ][4];
   for (int i = 0; i < n; ++i) {
-    const double rw = 1 / o.wq[i];
+    const double rw = div_rn(1.0, o.wq[i]);
     auto m = [&](int col) -> double {
       if (!limited) return o.MinvVhT[i + n * col];
       if (col < n) return col == i ? rw * 1.0 : 0.0;
@@ -865,7 +868,7 @@ __global__ void k_line_high(LineArgs a) {
       const double mm = m(n + f);
       for (int c = 0; c < 4; ++c) B[c] = B[c] + mm * BF[f][c];
     }
-    for (int c = 0; c < 4; ++c) rH[i][c] = -(A[c] + B[c]) / J;
+    for (int c = 0; c < 4; ++c) rH[i][c] = div_rn(-(A[c] + B[c]), J);
     st4(a.rhsH + 4 * ((size_t)n * k + i), rH[i]);
     ld4(a.rhsL + 4 * ((size_t)n * k + i), rL[i]);
     if (a.flags & LF_RHSU_H) st4(a.rhsU + 4 * ((size_t)n * k + i), rH[i]);
@@ -917,11 +920,11 @@ __global__ void k_line_high(LineArgs a) {
     stencil(q, kk, qq);
     Lphi[q] = 0.0;
     if (a.flags & LF_MINENT) {  // initialize_lower_bound!(::Dim1) (subcell.jl:37-51)
-      double lb = s_modified4(a.gamma, U[q]);
+      double lb = s_modified4(*a.ops, a.gamma, U[q]);
       for (int t = 0; t < 2; ++t) {
         double Un[4];
         ld4(a.Uq + 4 * ((size_t)n * kk[t] + qq[t]), Un);
-        lb = jmin(lb, s_modified4(a.gamma, Un));
+        lb = jmin(lb, s_modified4(*a.ops, a.gamma, Un));
       }
       Lphi[q] = epsk * lb + (1 - epsk) * phimin;
     }
@@ -956,7 +959,7 @@ __global__ void k_line_high(LineArgs a) {
   auto eval = [&](int q, int i, double sgn) {
     const double wJ = o.wq[q] * J;
     double P[4];
-    for (int c = 0; c < 4; ++c) P[c] = sgn * 2.0 * dt * (fH[i][c] - fL[i][c]) / wJ;
+    for (int c = 0; c < 4; ++c) P[c] = div_rn(sgn * 2.0 * dt * (fH[i][c] - fL[i][c]), wJ);
     const double Lrhoe = zeta * rhoe4(uL[q]);
     const double lpos = bound_rho_rhoe(uL[q], P, Lrho[q], Lrhoe, Urho[q], INFINITY, a.ZEROTOL);
     if (!(a.flags & LF_MINENT)) return lpos;
@@ -965,7 +968,7 @@ __global__ void k_line_high(LineArgs a) {
     auto okp = [&](double l) {
       double W[4];
       for (int c = 0; c < 4; ++c) W[c] = uL[q][c] + l * P[c];
-      return s_modified4(a.gamma, W) >= thr;
+      return s_modified4(*a.ops, a.gamma, W) >= thr;
     };
     double x_valid = 0.0, x_invalid = lpos;
     if (okp(x_invalid)) return x_invalid;
@@ -983,7 +986,7 @@ __global__ void k_line_high(LineArgs a) {
   for (int i = 0; i < 2 * n; ++i) L[i] = jmin(L[i], blend);
   if (a.flags & LF_CELL) {  // Dim1 methods of subcell.jl:468-505, 567-628, rhs_es :746-753
     double v[MQ][4];
-    for (int i = 0; i < n; ++i) v_ufun4(a.gamma, U[i], v[i]);
+    for (int i = 0; i < n; ++i) v_ufun4(*a.ops, a.gamma, U[i], v[i]);
     double sB = 0.0;
     for (int f = 0; f < 2; ++f) {
       double b0, b1;
@@ -1097,8 +1100,8 @@ __global__ void k_line_high_team(LineArgs a) {
     Bx(a, k, f, b0, b1);
     Bx(a, kP, iP, c0, c1);
     const double nn = norm2(b0, b1), nnP = norm2(c0, c1);
-    const double lam = wavespeed4(a.gamma, ut[n + f], b0 / nn, b1 / nn);
-    const double lamP = wavespeed4(a.gamma, uP[f], c0 / nnP, c1 / nnP);
+    const double lam = wavespeed4(a.gamma, ut[n + f], div_rn(b0, nn), div_rn(b1, nn));
+    const double lamP = wavespeed4(a.gamma, uP[f], div_rn(c0, nnP), div_rn(c1, nnP));
     LFc[f] = 0.5 * nn * jmax(lam, lamP);
     const int8_t bc = a.bc[fk];
     if (bc == BC_INFLOW || bc == BC_OUTFLOW) {
@@ -1144,7 +1147,7 @@ __global__ void k_line_high_team(LineArgs a) {
   const bool limited = th0 < 1.0 || th1 < 1.0;
   if (live && lane < n) {
     const int i = lane;
-    const double rw = 1 / o.wq[i];
+    const double rw = div_rn(1.0, o.wq[i]);
     auto m = [&](int col) -> double {
       if (!limited) return o.MinvVhT[i + n * col];
       if (col < n) return col == i ? rw * 1.0 : 0.0;
@@ -1162,7 +1165,7 @@ __global__ void k_line_high_team(LineArgs a) {
       const double mm = m(n + f);
       for (int c = 0; c < 4; ++c) B[c] = B[c] + mm * BF[f][c];
     }
-    for (int c = 0; c < 4; ++c) rH[i][c] = -(A[c] + B[c]) / J;
+    for (int c = 0; c < 4; ++c) rH[i][c] = div_rn(-(A[c] + B[c]), J);
     st4(a.rhsH + 4 * ((size_t)n * k + i), rH[i]);
     ld4(a.rhsL + 4 * ((size_t)n * k + i), rL[i]);
     if (a.flags & LF_RHSU_H) st4(a.rhsU + 4 * ((size_t)n * k + i), rH[i]);
@@ -1217,11 +1220,11 @@ __global__ void k_line_high_team(LineArgs a) {
     }
     Lphi[q] = 0.0;
     if (a.flags & LF_MINENT) {  // initialize_lower_bound!(::Dim1) (subcell.jl:37-51)
-      double lb = s_modified4(a.gamma, U[q]);
+      double lb = s_modified4(*a.ops, a.gamma, U[q]);
       for (int t = 0; t < 2; ++t) {
         double Un[4];
         ld4(a.Uq + 4 * ((size_t)n * kk[t] + qq[t]), Un);
-        lb = jmin(lb, s_modified4(a.gamma, Un));
+        lb = jmin(lb, s_modified4(*a.ops, a.gamma, Un));
       }
       Lphi[q] = epsk * lb + (1 - epsk) * phimin;
     }
@@ -1263,7 +1266,7 @@ __global__ void k_line_high_team(LineArgs a) {
     const double sgn = lane < n ? -1.0 : 1.0;
     const double wJ = o.wq[q] * J;
     double P[4];
-    for (int c = 0; c < 4; ++c) P[c] = sgn * 2.0 * dt * (fH[i][c] - fL[i][c]) / wJ;
+    for (int c = 0; c < 4; ++c) P[c] = div_rn(sgn * 2.0 * dt * (fH[i][c] - fL[i][c]), wJ);
     const double Lrhoe = zeta * rhoe4(uL[q]);
     double l = bound_rho_rhoe(uL[q], P, Lrho[q], Lrhoe, Urho[q], INFINITY, a.ZEROTOL);
     if (a.flags & LF_MINENT) {
@@ -1272,7 +1275,7 @@ __global__ void k_line_high_team(LineArgs a) {
       auto okp = [&](double lv) {
         double W[4];
         for (int c = 0; c < 4; ++c) W[c] = uL[q][c] + lv * P[c];
-        return s_modified4(a.gamma, W) >= thr;
+        return s_modified4(*a.ops, a.gamma, W) >= thr;
       };
       double x_valid = 0.0, x_invalid = l;
       if (!okp(x_invalid)) {
@@ -1300,7 +1303,7 @@ __global__ void k_line_high_team(LineArgs a) {
   __syncwarp();
   if (a.flags & LF_CELL) {  // Dim1 methods of subcell.jl:468-505, 567-628, rhs_es :746-753
     double(*v)[4] = sv[e];
-    if (live && lane < n) v_ufun4(a.gamma, U[lane], v[lane]);
+    if (live && lane < n) v_ufun4(*a.ops, a.gamma, U[lane], v[lane]);
     __syncwarp();
     if (live && lane == 0) {
       double sB = 0.0;
@@ -1395,7 +1398,7 @@ __global__ void k_line_update(LineArgs a) {
       for (int c = 0; c < 4; ++c) flim[i][c] = L[i] * fb[4 * i + c] + (1.0 - L[i]) * fb[4 * (n + 1 + i) + c];
     for (int i = 0; i < n; ++i) {
       const double wJ = o.wq[i] * J;
-      for (int c = 0; c < 4; ++c) rU[4 * i + c] = (flim[i + 1][c] - flim[i][c]) / wJ;
+      for (int c = 0; c < 4; ++c) rU[4 * i + c] = div_rn(flim[i + 1][c] - flim[i][c], wJ);
     }
   }
   if (!(a.flags & LF_UPDATE)) return;
@@ -1470,7 +1473,7 @@ __global__ void k_line_update_team(LineArgs a) {
       const int i = lane;
       const double wJ = o.wq[i] * J;
       for (int c = 0; c < 4; ++c) {
-        ru[c] = (flim[i + 1][c] - flim[i][c]) / wJ;
+        ru[c] = div_rn(flim[i + 1][c] - flim[i][c], wJ);
         rU[4 * i + c] = ru[c];
       }
     }

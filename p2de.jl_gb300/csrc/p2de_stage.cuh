@@ -39,6 +39,7 @@
 #include <stdint.h>
 
 #include "p2de_args.h"
+#include "p2de_arith.cuh"
 #include "p2de_physics.cuh"
 #include "p2de_tables.h"
 
@@ -123,114 +124,6 @@ struct Cfg {
 
 // U + dt rhsL, the low-order update (one form everywhere, so values agree bitwise)
 __device__ __forceinline__ double low_update(double u, double dt, double r) { return fma(dt, r, u); }
-
-// 1/x and sqrt(x) with most of the work off the FP64 pipe, which issues one warp instruction
-// per 17-20 clocks and SM here: an FP32 approximation (2^-23) is refined to about 44 bits in
-// FP32 and integer arithmetic (24-30 instructions on pipes that otherwise issue in a tenth of
-// their slots), and one FP64 Newton-Raphson step y + y (1 - x y), or for the root the step
-// g + (x - g g) y/2 from g = x y, y ~ 1/sqrt(x), gives the correctly rounded result unless it
-// lies within about 2^-88 relative of a rounding tie. 2 and 3 FP64 operations, 36 and 52 SM
-// clocks a warp; two Newton steps from the hardware's 20-bit FP64 reciprocal take 4 and 71
-// clocks, CUDA's square root 9 and 145. Compared on 8.6e9 arguments over the whole range: the
-// bits of __dsqrt_rn always, those of __drcp_rn but for mantissas of 53 ones (a tie to 2^-106,
-// where the two-step form rounds down too).
-//
-// seed_value: the double (y0 + v 2^-44) 2^-k for a float y0 in [1/2, 1], |v| < 2^22 and
-// sub = k << 20.
-__device__ __forceinline__ double seed_value(float y0, int v, int sub) {
-  const unsigned b = (unsigned)__float_as_int(y0);
-  const unsigned long long y =
-      ((unsigned long long)((b >> 3) + (896u << 20)) << 32 | (b << 29)) + (unsigned long long)(long long)(v * 512);
-  return __hiloint2double((int)(y >> 32) - sub, (int)(unsigned)y);
-}
-// the 29 mantissa bits of a double below its leading 24, cut to 23, as a float in [0, 1) 2^s
-// for the float exponent bits eb = (127 + s) << 23
-__device__ __forceinline__ float low_bits(unsigned lo, int eb) {
-  return __fsub_rn(__int_as_float((int)((lo >> 6) & 0x7fffffu) | eb), __int_as_float(eb));
-}
-constexpr float kSeedMagic = 12582912.0f;  // 1.5 2^23: the low mantissa bits of x + this are x as an integer
-
-// 1/x for |x| in [2^-1021, 2^1021); other x take __drcp_rn
-__device__ __forceinline__ double rcp(double x) {
-  const int hi = __double2hiint(x);
-  const unsigned lo = (unsigned)__double2loint(x);
-  if ((unsigned)((hi & 0x7fffffff) - 0x00200000) >= 0x7fa00000u) return __drcp_rn(x);
-  const float xh = __int_as_float((int)(__funnelshift_l(lo, (unsigned)hi, 3) & 0x7fffffu) | 0x3f800000);
-  const float xl = low_bits(lo, 0x3f800000);
-  float y0;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(xh));
-  float e = __fmaf_rn(-xh, y0, 1.0f);
-  e = __fmaf_rn(__fmul_rn(y0, -0x1p-23f), xl, e);  // 1 - x y0
-  const int v = __float_as_int(__fmaf_rn(__fmul_rn(y0, 0x1p44f), e, kSeedMagic)) - 0x4b400000;
-  double y = seed_value(y0, v, (hi & 0x7ff00000) - (1023 << 20));
-  y = __hiloint2double(__double2hiint(y) | (hi & (int)0x80000000), __double2loint(y));
-  return __fma_rn(y, __fma_rn(-x, y, 1.0), y);
-}
-
-// sqrt(x) for x in [2^-900, 2^900]; other x take __dsqrt_rn
-__device__ __forceinline__ double sqrt_rn(double x) {
-  const int hi = __double2hiint(x);
-  const unsigned lo = (unsigned)__double2loint(x);
-  if ((unsigned)(hi - (123 << 20)) >= (1800u << 20)) return __dsqrt_rn(x);
-  // x = m 4^k with m in [1, 4)
-  const int mb = (int)((__funnelshift_l(lo, (unsigned)hi, 3) & 0xffffffu) ^ 0x800000u) + 0x3f800000;
-  const float xh = __int_as_float(mb), xl = low_bits(lo, mb & 0x7f800000);
-  const int k20 = ((hi - (1023 << 20)) >> 1) & (int)0xfff00000;  // k << 20
-  float y0;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(xh));
-  const float th = __fmul_rn(y0, y0), tl = __fmaf_rn(y0, y0, -th);
-  float e = __fmaf_rn(-xh, th, 1.0f);
-  e = __fmaf_rn(-xh, tl, e);
-  e = __fmaf_rn(__fmul_rn(th, -0x1p-23f), xl, e);  // 1 - m y0^2
-  const int v = __float_as_int(__fmaf_rn(__fmul_rn(y0, 0x1p43f), e, kSeedMagic)) - 0x4b400000;
-  const double y = seed_value(y0, v, k20);
-  const double g = __dmul_rn(x, y);
-  const double h = __hiloint2double(__double2hiint(y) - (1 << 20), __double2loint(y));
-  return __fma_rn(__fma_rn(-g, g, x), h, g);
-}
-
-// Natural logarithm by the table-driven method of P. T. P. Tang ("Table-driven implementation
-// of the logarithm function in IEEE floating-point arithmetic", ACM TOMS 16(4), 1990):
-// x = 2^k m with m in [sqrt(1/2), sqrt(2)), F = m rounded to a multiple of 1/256 (table
-// entry j), r = (m - F) / F (m - F exact), log x = k log 2 + log F + log(1 + r), the last
-// by its Taylor polynomial to r^6 (|r| < 2^-8.5: the omitted terms are below 2^-56 of the
-// result). 15 FP64 instructions against 31 for log(); within one unit in the last place of
-// the correctly rounded value (checked against an extended-precision log on 4M arguments
-// from 1e-9 to 2e8 and around 1), like log(). Positive normal finite x; anything else
-// goes to log(). HALF: log(x/2), the same bits as log_fast(0.5 x) (the halving is in the
-// exponent).
-template <bool HALF = false>
-__device__ __forceinline__ double log_fast(double x, const OpTable& op) {
-  const long long b = __double_as_longlong(x);
-  if ((unsigned long long)(b - (HALF ? 0x0020000000000000LL : 0x0010000000000000LL)) >=
-      (HALF ? 0x7fd0000000000000ULL : 0x7fe0000000000000ULL))
-    return log(HALF ? 0.5 * x : x);
-  long long k = (b >> 52) - (HALF ? 1024 : 1023);
-  long long mb = (b & 0x000fffffffffffffLL) | 0x3ff0000000000000LL;  // m in [1, 2)
-  if (((mb >> 44) & 0xff) >= 106) {  // m >= 1 + 106/256: use m/2 in [0.707, 1)
-    mb -= 0x0010000000000000LL;
-    k += 1;
-  }
-  const double m = __longlong_as_double(mb);
-  // F = m rounded to a multiple of 2^-8, on the integer pipe: the exponent field is 1023 (m in
-  // [1, sqrt 2)) or 1022
-  const int mh = (int)(mb >> 32), sh = 13 - (mh >> 20 & 1);
-  const int Fh = ((mh >> (sh - 1)) + 1) >> 1;  // F in units of 2^-7 or 2^-8 above its binade
-  const double F = __hiloint2double(Fh << sh, 0);
-  const int j = Fh - (sh == 12 ? (0x3ff00000 >> 12) - 256 : (0x3fe00000 >> 13) - 128);
-  const double* T = op.logtab[j - kLogTabLo];
-  const double r = (m - F) * T[0];
-  double q = fma(r, -1.0 / 6.0, 1.0 / 5.0);
-  q = fma(q, r, -0.25);
-  q = fma(q, r, 1.0 / 3.0);
-  q = fma(q, r, -0.5);
-  const double p = fma(r * r, q, r);
-  // (double)k without a conversion: 1.5 2^52 + k in the bits of 1.5 2^52, minus 1.5 2^52
-  const double kd = __longlong_as_double(0x4338000000000000LL + k) - 0x1.8p52;
-  const double hi = fma(kd, op.ln2_hi, T[1]);
-  const double lo = fma(kd, op.ln2_lo, T[2]);
-  return hi + (p + lo);
-}
 
 // Geometry factor q of an element from gg = (J, rxJ, sxJ, ryJ, syJ): slots 0-4 copy gg,
 // then |gr|, nr (2), |gs|, ns (2), 1/J; slots 12-14 hold FP32 rxJ, sxJ, ryJ, syJ, 1/J
@@ -586,13 +479,13 @@ __device__ __forceinline__ int& bisect_slot(double* sm, int PE, int s) {
 
 // v_ufun(::CompressibleIdealGas{Dim2}) (compressible_Navier_Stokes.jl:134-144), with
 // s = log(p) - gamma log(rho) for log(p / rho^gamma)
-__device__ __forceinline__ void v_ufun_d(const Gas<double>& g, const double* U, double* V) {
-  const double p = g.gm1 * (U[3] - 0.5 * (U[1] * U[1] + U[2] * U[2]) / U[0]);
-  const double s = log(p) - g.gamma * log(U[0]);
-  V[0] = (g.gamma + 1.0 - s) - g.gm1 * U[3] / p;
-  V[1] = U[1] * g.gm1 / p;
-  V[2] = U[2] * g.gm1 / p;
-  V[3] = -U[0] * g.gm1 / p;
+__device__ __forceinline__ void v_ufun_d(const Gas<double>& g, const double* U, double* V, const OpTable& op) {
+  const double p = g.gm1 * (U[3] - div_rn(0.5 * (U[1] * U[1] + U[2] * U[2]), U[0]));
+  const double s = log_fast(p, op) - g.gamma * log_fast(U[0], op);
+  V[0] = (g.gamma + 1.0 - s) - div_rn(g.gm1 * U[3], p);
+  V[1] = div_rn(U[1] * g.gm1, p);
+  V[2] = div_rn(U[2] * g.gm1, p);
+  V[3] = div_rn(-U[0] * g.gm1, p);
 }
 
 // v_ufun_d with every operation an explicit round-to-nearest intrinsic: the compiler cannot
@@ -612,10 +505,11 @@ __device__ __forceinline__ void v_ufun_rn(const Gas<double>& g, const double* U,
 // rhoe_vfun = ((gamma-1) / (-vE)^gamma)^(1/(gamma-1)) exp(-s/(gamma-1)) is evaluated as the
 // one exponential exp((log(gamma-1) - gamma log(-vE) - s) / (gamma-1)) (the same value to
 // about 1e-14 relative; two pow calls fewer); lgm1 = log(gamma - 1).
-__device__ __forceinline__ void u_vfun_d(const Gas<double>& g, double lgm1, const double* V, double* U) {
-  const double q = (V[1] * V[1] + V[2] * V[2]) / (2.0 * V[3]);
+__device__ __forceinline__ void u_vfun_d(const Gas<double>& g, double lgm1, const double* V, double* U,
+                                         const OpTable& op) {
+  const double q = div_rn(V[1] * V[1] + V[2] * V[2], 2.0 * V[3]);
   const double s = g.gamma - V[0] + q;
-  const double rhoeV = exp((lgm1 - g.gamma * log(-V[3]) - s) / g.gm1);
+  const double rhoeV = exp_fast(div_rn(lgm1 - g.gamma * log_fast(-V[3], op) - s, g.gm1), op);
   U[0] = -rhoeV * V[3];
   U[1] = rhoeV * V[1];
   U[2] = rhoeV * V[2];
@@ -648,7 +542,7 @@ __device__ __forceinline__ void gauss_proj_body(const StageArgs& a, int k0, doub
   __syncthreads();
   for (int w = tid; w < Ke * Nq; w += bs) {
     const int e = w / Nq, m = w % Nq;
-    v_ufun_d(g, sm + e * PE + 4 * m, sm + e * PE + 4 * Nq + 4 * m);
+    v_ufun_d(g, sm + e * PE + 4 * m, sm + e * PE + 4 * Nq + 4 * m, op);
   }
   __syncthreads();
   const double eps = a.POSTOL, lgm1 = log(a.gm1);
@@ -672,7 +566,7 @@ __device__ __forceinline__ void gauss_proj_body(const StageArgs& a, int k0, doub
         VUf[c] = VUf[c] + ell[i] * vq[4 * node[i] + c];
       }
     }
-    const double rhoef = Uf[3] - 0.5 * (Uf[1] * Uf[1] + Uf[2] * Uf[2]) / Uf[0];
+    const double rhoef = Uf[3] - div_rn(0.5 * (Uf[1] * Uf[1] + Uf[2] * Uf[2]), Uf[0]);
     auto project = [&](double th, double* vt) {
 #pragma unroll
       for (int c = 0; c < 4; ++c) vt[c] = 0.0;
@@ -688,8 +582,8 @@ __device__ __forceinline__ void gauss_proj_body(const StageArgs& a, int k0, doub
     auto ok = [&](double th) {
       project(th, vt);
       if (!(vt[3] < -eps)) return false;
-      u_vfun_d(g, lgm1, vt, ut);
-      const double rhoe = ut[3] - 0.5 * (ut[1] * ut[1] + ut[2] * ut[2]) / ut[0];
+      u_vfun_d(g, lgm1, vt, ut, op);
+      const double rhoe = ut[3] - div_rn(0.5 * (ut[1] * ut[1] + ut[2] * ut[2]), ut[0]);
       return vt[3] < fmin(a.zeta * VUf[3], -eps) && ut[0] > fmax((1 - a.eta) * Uf[0], eps) &&
              ut[0] < (1 + a.eta) * Uf[0] && rhoe > fmax((1 - a.eta) * rhoef, eps) && rhoe < (1 + a.eta) * rhoef;
     };
@@ -712,7 +606,7 @@ __device__ __forceinline__ void gauss_proj_body(const StageArgs& a, int k0, doub
     }
     if (!have) {
       project(th, vt);
-      u_vfun_d(g, lgm1, vt, ut);
+      u_vfun_d(g, lgm1, vt, ut, op);
     }
 #pragma unroll
     for (int c = 0; c < 4; ++c) a.ufproj[((size_t)k * Nfp + f) * 4 + c] = ut[c];

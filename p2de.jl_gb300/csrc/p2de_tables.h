@@ -68,6 +68,9 @@ struct OpTable {
   // the same two parts (42 significant bits, so that k log2_hi is exact for |k| < 2048)
   double logtab[kLogTabN][3];
   double ln2_hi, ln2_lo;
+  // exp_fast: 2^(j/128) in two parts, 128/log 2, log 2/128 to 35 bits and the rest
+  double exptab[128][2];
+  double exp_inv, exp_hi, exp_lo;
   // flux form (p2de_flux.cuh): 1/w1D, and per high-order pair -hp_S / w of its line's
   // tangential weight w (FP64, FP32)
   double rw1D[kMaxN1D];
@@ -92,6 +95,11 @@ struct LineOps {
   int8_t pi[kLineMaxPairs], pj[kLineMaxPairs];  // its nonzero pairs i > j, j outer (init.jl:188-195)
   double MinvVhT[kMaxN1D * kLineMaxNh];   // M \ Vh' = (1/wq) [I, Vf'], column-major Nq x Nh
   double VDMinv[kMaxN1D * kMaxN1D];       // inv(VDM) of the orthonormal Legendre modes, row-major
+  double logtab[kLogTabN][3];             // log_fast, as in OpTable
+  double ln2_hi, ln2_lo;
+  // exp_fast: 2^(j/128) in two parts, 128/log 2, log 2/128 to 35 bits and the rest
+  double exptab[128][2];
+  double exp_inv, exp_hi, exp_lo;
 };
 
 // Builds the Line operators for degree N (1..5) on LGL (basis 0) or Gauss (basis 1) nodes.
