@@ -71,29 +71,29 @@ static size_t smem_a_of(int epb, int kind) {
   switch (kind) {
     case BATCH_PLAIN: return Cfg<N1D>::smem_a(epb);
     case BATCH_EXT: return Cfg<N1D>::smem_x(epb);
-    case BATCH_FLUX: return FluxCfg<N1D>::template smem<false>(epb);
+    case BATCH_FLUX: return FluxCfg<N1D>::template smem<false, true>(epb);
     default: return FluxCfg<N1D>::template smem<true>(epb);
   }
 }
 
 int batch_elems_per_block(int n1d, bool flux) {
   switch (n1d) {
-    case 2: return flux ? FluxCfg<2>::E : Cfg<2>::E;
-    case 3: return flux ? FluxCfg<3>::E : Cfg<3>::E;
-    case 4: return flux ? FluxCfg<4>::E : Cfg<4>::E;
-    case 5: return flux ? FluxCfg<5>::E : Cfg<5>::E;
-    case 6: return flux ? FluxCfg<6>::E : Cfg<6>::E;
+    case 2: return flux ? FluxCfg<2>::E_BATCH : Cfg<2>::E;
+    case 3: return flux ? FluxCfg<3>::E_BATCH : Cfg<3>::E;
+    case 4: return flux ? FluxCfg<4>::E_BATCH : Cfg<4>::E;
+    case 5: return flux ? FluxCfg<5>::E_BATCH : Cfg<5>::E;
+    case 6: return flux ? FluxCfg<6>::E_BATCH : Cfg<6>::E;
   }
   return 0;
 }
 
 int batch_elems_per_block_max(int n1d) {
   switch (n1d) {
-    case 2: return cmin(Cfg<2>::E_MAX, FluxCfg<2>::E_MAX);
-    case 3: return cmin(Cfg<3>::E_MAX, FluxCfg<3>::E_MAX);
-    case 4: return cmin(Cfg<4>::E_MAX, FluxCfg<4>::E_MAX);
-    case 5: return cmin(Cfg<5>::E_MAX, FluxCfg<5>::E_MAX);
-    case 6: return cmin(Cfg<6>::E_MAX, FluxCfg<6>::E_MAX);
+    case 2: return cmin(Cfg<2>::E_MAX, FluxCfg<2>::E_SPLIT_MAX);
+    case 3: return cmin(Cfg<3>::E_MAX, FluxCfg<3>::E_SPLIT_MAX);
+    case 4: return cmin(Cfg<4>::E_MAX, FluxCfg<4>::E_SPLIT_MAX);
+    case 5: return cmin(Cfg<5>::E_MAX, FluxCfg<5>::E_SPLIT_MAX);
+    case 6: return cmin(Cfg<6>::E_MAX, FluxCfg<6>::E_SPLIT_MAX);
   }
   return 0;
 }

@@ -39,9 +39,9 @@ constexpr size_t kBatchSmemXMax =
          Cfg<6>::smem_x(Cfg<6>::E_MAX));
 template <bool EXT>
 constexpr size_t kBatchSmemFluxMax =
-    smax(smax(smax(FluxCfg<2>::smem<EXT>(FluxCfg<2>::E_MAX), FluxCfg<3>::smem<EXT>(FluxCfg<3>::E_MAX)),
-              smax(FluxCfg<4>::smem<EXT>(FluxCfg<4>::E_MAX), FluxCfg<5>::smem<EXT>(FluxCfg<5>::E_MAX))),
-         FluxCfg<6>::smem<EXT>(FluxCfg<6>::E_MAX));
+    smax(smax(smax(FluxCfg<2>::smem<EXT, !EXT>(FluxCfg<2>::E_SPLIT_MAX), FluxCfg<3>::smem<EXT, !EXT>(FluxCfg<3>::E_SPLIT_MAX)),
+              smax(FluxCfg<4>::smem<EXT, !EXT>(FluxCfg<4>::E_SPLIT_MAX), FluxCfg<5>::smem<EXT, !EXT>(FluxCfg<5>::E_SPLIT_MAX))),
+         FluxCfg<6>::smem<EXT, !EXT>(FluxCfg<6>::E_SPLIT_MAX));
 constexpr size_t kBatchSmemBMax =
     smax(smax(smax(Cfg<2>::smem_b(Cfg<2>::E_MAX), Cfg<3>::smem_b(Cfg<3>::E_MAX)),
               smax(Cfg<4>::smem_b(Cfg<4>::E_MAX), Cfg<5>::smem_b(Cfg<5>::E_MAX))),
@@ -106,7 +106,10 @@ __global__ void __launch_bounds__(kBatchThreads) k_batch_a(const StageArgs* solv
   }
 }
 
-// the members whose stage kernels run in flux form (p2de_flux.cuh)
+// the members whose stage kernels run in flux form (p2de_flux.cuh). Blocks of 128 threads run
+// the lines split over their warps (FluxLine): one thread a line would leave three of a
+// block's four warps idle there (DMR 480x120 N=3, 4 elements a block, as one solve: 745 us a
+// stage with one thread a line, 645 split).
 template <typename TH, bool EXT>
 __global__ void __launch_bounds__(kBatchThreads) k_batch_flux_a(const StageArgs* solves, const BatchTask* tasks,
                                                                 const int* ntasks, unsigned* counter, int nstage,
@@ -117,11 +120,11 @@ __global__ void __launch_bounds__(kBatchThreads) k_batch_flux_a(const StageArgs*
   BatchTask tk;
   while (batch_next(solves, tasks, ntasks, counter, nstage, sa, tk, s_task, mode)) {
     switch (tk.n1d) {
-      case 2: flux_a_body<2, TH, EXT>(sa, tk.k0, sm); break;
-      case 3: flux_a_body<3, TH, EXT>(sa, tk.k0, sm); break;
-      case 4: flux_a_body<4, TH, EXT>(sa, tk.k0, sm); break;
-      case 5: flux_a_body<5, TH, EXT>(sa, tk.k0, sm); break;
-      case 6: flux_a_body<6, TH, EXT>(sa, tk.k0, sm); break;
+      case 2: flux_a_body<2, TH, EXT, !EXT>(sa, tk.k0, sm); break;
+      case 3: flux_a_body<3, TH, EXT, !EXT>(sa, tk.k0, sm); break;
+      case 4: flux_a_body<4, TH, EXT, !EXT>(sa, tk.k0, sm); break;
+      case 5: flux_a_body<5, TH, EXT, !EXT>(sa, tk.k0, sm); break;
+      case 6: flux_a_body<6, TH, EXT, !EXT>(sa, tk.k0, sm); break;
     }
   }
 }

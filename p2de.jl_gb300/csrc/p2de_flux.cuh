@@ -65,6 +65,8 @@ struct FluxCfg {
   static constexpr int THREADS = 128;
   // default elements per block: lines and nodes in (nearly) full warps
   static constexpr int E = n == 2 ? 16 : n == 3 ? 10 : n == 4 ? 4 : n == 5 ? 6 : 5;
+  // and in the batched kernel (split lines, 128 threads)
+  static constexpr int E_BATCH = n == 2 ? 16 : n == 3 ? 5 : n == 4 ? 4 : n == 5 ? 3 : 2;
   // shared-memory doubles per element; arrays over nodes and faces are component-major
   static constexpr int O_C = 0;                 // 6n: cx, cy; s = 4 dt c of both; 1/s of both
   static constexpr int O_U = O_C + 6 * n;       // 4 Nq: state
@@ -104,7 +106,7 @@ struct FluxCfg {
   static constexpr int E_SPLIT_RAW =
       (int)((224 * 1024 - 64) / (sizeof(double) * Lay<false, true>::PE + sizeof(int) * NF));
   static constexpr int E_SPLIT_MAX = E_SPLIT_RAW < 32 ? E_SPLIT_RAW : 32;
-  static_assert(E <= E_MAX, "flux layout");
+  static_assert(E <= E_MAX && E_BATCH <= E_SPLIT_MAX && E_SPLIT_MAX <= E_MAX, "flux layout");
 };
 
 // fS(Dim2) (compressible_Navier_Stokes.jl:220-249) along axis ax for line nodes a and b, in
