@@ -287,6 +287,16 @@ class Solver:
         self._check(self.lib.p2de_get_field(self.handle, field, nstage, abi.dptr(out)))
         return out
 
+    def read_field(self, field: int, out: np.ndarray, nstage: int = 1) -> None:
+        """A field copied into an existing array: straight from the device when the array is
+        contiguous float64 (no temporary of the field's size, no second copy), else through
+        get_field."""
+        if (out.dtype == np.float64 and out.flags.c_contiguous and out.flags.writeable
+                and out.size == self.field_count(field)):
+            self._check(self.lib.p2de_get_field(self.handle, field, nstage, abi.dptr(out)))
+        else:
+            out[...] = self.get_field(field, nstage).reshape(out.shape)
+
     def set_Uq(self, Uq: np.ndarray) -> None:
         U = np.ascontiguousarray(Uq, dtype=np.float64)
         if U.size != self.field_count(abi.FIELD_UQ):
@@ -428,11 +438,10 @@ def rhs_bang(state, solver: Solver, state_param: StateParam, time_param: TimePar
     solver._check(solver.lib.p2de_rhs(solver.handle, time_param.t, time_param.dt, time_param.nstage, byref(out)))
     if host:
         pre = state.preallocation
-        pre.rhsU[...] = solver.get_field(abi.FIELD_RHSU).reshape(pre.rhsU.shape)
+        solver.read_field(abi.FIELD_RHSU, pre.rhsU)
         lim = solver.param.rhs_limiter
         if isinstance(solver.param.rhs, ESLimitedLowOrderPos) and isinstance(lim, SubcellLimiter):
-            s = time_param.nstage - 1
-            pre.L_local[s] = solver.get_field(abi.FIELD_L_LOCAL, time_param.nstage).reshape(pre.L_local[s].shape)
+            solver.read_field(abi.FIELD_L_LOCAL, pre.L_local[time_param.nstage - 1], time_param.nstage)
     return out.value
 
 
