@@ -37,15 +37,6 @@ __device__ __forceinline__ double dsub(double a, double b) { return __dsub_rn(a,
 __device__ __forceinline__ double dmul(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double dfma(double a, double b, double c) { return __fma_rn(a, b, c); }
 
-// x/2 and 2x on the integer pipe: a step of the exponent where x and the result are normal
-__device__ __forceinline__ double scale_exponent(double x, int step) {
-  const int hi = __double2hiint(x), ef = hi & 0x7ff00000;
-  if ((unsigned)(ef - 0x00200000) < 0x7fb00000u) return __hiloint2double(hi + step, __double2loint(x));
-  return is_zero_bits(x) ? x : __dmul_rn(step < 0 ? 0.5 : 2.0, x);
-}
-__device__ __forceinline__ double half(double x) { return scale_exponent(x, -0x00100000); }
-__device__ __forceinline__ double twice(double x) { return scale_exponent(x, 0x00100000); }
-
 __device__ __forceinline__ bool negative(double x) { return __double2hiint(x) < 0; }
 // > 0 and not NaN, by the bits
 __device__ __forceinline__ bool positive_bits(double x) {
@@ -115,20 +106,9 @@ struct FluxCfg {
 // sum where they settle it (all but two of them), else as written. In its series branch
 // x = da/aavg has x^2 < 1e-8, so the x^4 and x^6 terms of the series (and of its reciprocal,
 // for betalog) are below 2^-53 and are not formed.
-// |x| in [2^-999, 2^1000)
-__device__ __forceinline__ bool mid_exponent(double x) {
-  return (unsigned)((__double2hiint(x) & 0x7ff00000) - (24 << 20)) < (1999u << 20);
-}
 struct PairState {
   double rho, vn, vt, hn, ht, beta, lr, lb;  // velocities normal and tangential to the axis, and halves
 };
-__device__ __forceinline__ bool series_branch(double d, double s) {
-  const int ed = (__double2hiint(d) >> 20) & 0x7ff, es = (__double2hiint(s) >> 20) & 0x7ff;
-  const int k = ed - es;  // |d|/s in (2^(k-1), 2^(k+1)); the line lies at |d| < 0.5e-4 s
-  if (k >= -13) return false;
-  if (k <= -16) return true;
-  return fabs(d) < 1e-4 * fabs(0.5 * s);
-}
 __device__ __forceinline__ void fS_line(double ig, const PairState& a, const PairState& b, double* F0, double* Ft,
                                         double* Fn, double* F3) {
   const double sr = dadd(a.rho, b.rho), dr = dsub(b.rho, a.rho);

@@ -14,6 +14,7 @@ struct Gas {
   T gamma;   // gamma
   T gm1;     // gamma - 1.0 (computed once on the host as the reference does at run time)
   T two_gm1; // 2 * (gamma - 1)
+  T rtwo_gm1; // 1 / (2 (gamma - 1)) (FP64 two-point flux)
 };
 
 // pfun (:24-28)

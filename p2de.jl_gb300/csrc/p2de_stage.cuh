@@ -173,6 +173,15 @@ __device__ __forceinline__ float signed_by(float x, int sign) {
 // x == +-0 by its bits (integer pipe instead of the FP64 pipe)
 __device__ __forceinline__ bool is_zero_bits(double x) { return (__double_as_longlong(x) << 1) == 0; }
 
+// x/2 and 2x on the integer pipe: a step of the exponent where x and the result are normal
+__device__ __forceinline__ double scale_exponent(double x, int step) {
+  const int hi = __double2hiint(x), ef = hi & 0x7ff00000;
+  if ((unsigned)(ef - 0x00200000) < 0x7fb00000u) return __hiloint2double(hi + step, __double2loint(x));
+  return is_zero_bits(x) ? x : __dmul_rn(step < 0 ? 0.5 : 2.0, x);
+}
+__device__ __forceinline__ double half(double x) { return scale_exponent(x, -0x00100000); }
+__device__ __forceinline__ double twice(double x) { return scale_exponent(x, 0x00100000); }
+
 // min of two values in [0, Inf] (either zero's sign) or NaN, by their magnitude bits: a
 // NaN loses against any number, as with fmin; the result of a zero is +0
 __device__ __forceinline__ double min_nonneg_bits(double a, double b) {
@@ -277,20 +286,64 @@ __device__ __forceinline__ void fS_fast(const Gas<double>& g, const double* UL, 
   Fy[3] = c.f4aux * c.vavg;
 }
 
-// the x (ax = 0) or y (ax = 1) flux of fS_fast alone, with the same operations for each
-// component: on axis-aligned elements a pair on an r-line needs only the x flux and a pair
-// on an s-line only the y flux, and one instruction stream serves both
+// |x| in [2^-999, 2^1000)
+__device__ __forceinline__ bool mid_exponent(double x) {
+  return (unsigned)((__double2hiint(x) & 0x7ff00000) - (24 << 20)) < (1999u << 20);
+}
+// The log mean's branch test |d/(s/2)| < 1e-4 for d = aR - aL, s = aL + aR: decided from the
+// exponents where they settle it (all but two of their differences), else as written.
+__device__ __forceinline__ bool series_branch(double d, double s) {
+  const int ed = (__double2hiint(d) >> 20) & 0x7ff, es = (__double2hiint(s) >> 20) & 0x7ff;
+  const int k = ed - es;  // |d|/s in (2^(k-1), 2^(k+1)); the line lies at |d| < 0.5e-4 s
+  if (k >= -13) return false;
+  if (k <= -16) return true;
+  return fabs(d) < 1e-4 * fabs(0.5 * s);
+}
+
+// the x (ax = 0) or y (ax = 1) flux of fS alone (compressible_Navier_Stokes.jl:220-249): on
+// axis-aligned elements a pair on an r-line needs only the x flux and a pair on an s-line only
+// the y flux, and one instruction stream serves both. One reciprocal gives 1/(betaL + betaR)
+// and the quotients of both log means; in the series branch x = da/aavg has x^2 < 1e-8, so the
+// series' later terms (and its reciprocal's, for betalog) are below 2^-53 and are not formed;
+// halvings step the exponent. 36 FP64 operations against 51 for fS_fast's order.
 __device__ __forceinline__ void fS_axis(const Gas<double>& g, const double* UL, const double* UR, int ax,
                                         double* F) {
-  const FSCommon c = fS_common(g, UL, UR);
-  const double un = ax ? c.vavg : c.uavg;
-  const double F0 = c.rholog * un;                 // FxS1 or FyS1
-  const double Ft = (c.rholog * c.uavg) * c.vavg;  // FxS3: Fx[2] and Fy[1]
-  const double Fn = fma(F0, un, c.pa);             // Fx[1] or Fy[2]
+  const double sr = UL[0] + UR[0], dr = UR[0] - UL[0], sb = UL[3] + UR[3], db = UR[3] - UL[3];
+  const bool ser_r = series_branch(dr, sr), ser_b = series_branch(db, sb);
+  const double den_r = ser_r ? sr : UL[4] - UR[4], den_b = ser_b ? sb : db;
+  const double t = den_r * den_b, D = t * sb;
+  double isb, idr, idb;  // 1/sb, 1/den_r, 1/den_b
+  if (mid_exponent(t) && mid_exponent(D)) {
+    const double r = rcp(D), q = sb * r;
+    isb = t * r;
+    idr = den_b * q;
+    idb = den_r * q;
+  } else {  // the products leave the range of doubles
+    isb = rcp(sb);
+    idr = rcp(den_r);
+    idb = rcp(den_b);
+  }
+  const double x = dr * idr;
+  double rl = -x;               // rho log mean
+  double nb = UR[5] - UL[5];    // numerator of 1/beta log mean
+  if (ser_r) rl = sr * fma(x * x, -0.4, 0.5);
+  if (ser_b) {
+    const double y = db * isb;
+    nb = fma(y * y, 1.6, 2.0);
+  }
+  const double ilb = nb * idb;
+  const double pa = half(sr) * isb;
+  const double ua = half(UL[1] + UR[1]), va = half(UL[2] + UR[2]);
+  const double unorm = fma(UL[1], UR[1], UL[2] * UR[2]);
+  const double f4aux = fma(rl * ilb, g.rtwo_gm1, fma(half(rl), unorm, pa));
+  const double un = ax ? va : ua;
+  const double F0 = rl * un;
+  const double Ft = F0 * (ax ? ua : va);  // the tangential momentum flux
+  const double Fn = fma(F0, un, pa);
   F[0] = F0;
   F[1] = ax ? Ft : Fn;
   F[2] = ax ? Fn : Ft;
-  F[3] = c.f4aux * un;
+  F[3] = f4aux * un;
 }
 
 // limiter_utils.jl:108-132 for a finite Lrhoe
@@ -385,16 +438,49 @@ __device__ __forceinline__ void fS_kpp(double uL, double uR, double* Fx, double*
 }
 
 // find_alpha(::CompressibleIdealGas) (low_order_graph_viscosity.jl:316-340): doubling, then
-// 50 halvings toward the alpha with alpha ui - uitilde of positive density and rhoe
+// 50 halvings toward the alpha with alpha ui - uitilde of positive density and rhoe. The valid
+// alphas are an upper interval (the states of positive density and rhoe are a convex cone that
+// holds ui), so the halvings end at the smallest valid multiple of alphaR 2^-50. Its place
+// comes from the bounds' closed form in beta = alpha - 1 (q = beta ui + d, d = ui - uitilde, so
+// nothing cancels for nearly equal states), and the reference's test is made at that multiple
+// and its neighbours; the halvings run where that does not settle it within a few steps. 12
+// tests at most against 51 (Sedov 80x80 N=3, stage 1: kernel A 504 us with the halvings).
 __device__ __forceinline__ double find_alpha(const double* ui, const double* ut, double POSTOL) {
   auto ok = [&](double al) {
     double q[4];
 #pragma unroll
     for (int c = 0; c < 4; ++c) q[c] = al * ui[c] - ut[c];
-    return q[0] > POSTOL && q[3] - 0.5 * (q[1] * q[1] + q[2] * q[2]) / q[0] > POSTOL;
+    return q[0] > POSTOL && q[3] - div_rn(0.5 * (q[1] * q[1] + q[2] * q[2]), q[0]) > POSTOL;
   };
   double alphaL = 0.0, alphaR = 1.0;
   for (int guard = 0; guard < 1100 && !ok(alphaR); ++guard) alphaR = 2 * alphaR;
+  {
+    double d[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) d[c] = ui[c] - ut[c];
+    // density: beta ui0 + d0 > POSTOL; rhoe: A beta^2 + B beta + C > 0
+    const double A = fma(ui[3], ui[0], -0.5 * fma(ui[1], ui[1], ui[2] * ui[2]));
+    const double B = fma(ui[3], d[0], fma(d[3] - POSTOL, ui[0], -fma(ui[1], d[1], ui[2] * d[2])));
+    const double C = fma(d[3] - POSTOL, d[0], -0.5 * fma(d[1], d[1], d[2] * d[2]));
+    const double rA = rcp(A + A), sq = sqrt_rn(fmax(fma(B, B, -4.0 * A * C), 0.0));
+    const double beta = fmax(div_rn(POSTOL - d[0], ui[0]), (sq - B) * rA);
+    const double step = alphaR * 0x1p-50;
+    double al = ceil((1.0 + beta) * (0x1p50 / alphaR)) * step;
+    if (al > 0.0 && al <= alphaR) {
+      int left = 6;
+      while (left > 0 && !ok(al)) {
+        al += step;
+        --left;
+      }
+      bool at = false;
+      while (left > 0 && !at) {
+        at = !ok(al - step);
+        if (!at) al -= step;
+        --left;
+      }
+      if (at) return al;
+    }
+  }
   for (int iter = 0; iter < 50; ++iter) {
     const double alphaM = (alphaL + alphaR) / 2;
     if (ok(alphaM))
@@ -534,7 +620,7 @@ __device__ __forceinline__ void gauss_proj_body(const StageArgs& a, int k0, doub
   const int tid = threadIdx.x, bs = blockDim.x;
   const int Ke = min(a.epb, a.K - k0);
   if (Ke <= 0) return;
-  const Gas<double> g{a.gamma, a.gm1, 2.0 * a.gm1};
+  const Gas<double> g{a.gamma, a.gm1, 2.0 * a.gm1, 0.5 * a.rgm1};
   for (int w = tid; w < Ke * Nq * 4; w += bs) {
     const int e = w / (Nq * 4), r = w % (Nq * 4);
     sm[e * PE + r] = a.Uq[(size_t)k0 * Nq * 4 + w];
@@ -629,7 +715,7 @@ __device__ __forceinline__ void es_interface_body(const StageArgs& a, long long 
   if (a.scal[S_DONE] != 0.0) return;
   if (w >= (long long)a.K * Nfp) return;
   const OpTable& op = *a.ops;
-  const Gas<double> g{a.gamma, a.gm1, 2.0 * a.gm1};
+  const Gas<double> g{a.gamma, a.gm1, 2.0 * a.gm1, 0.5 * a.rgm1};
   const int k = (int)(w / Nfp), f = (int)(w % Nfp);
   const int lin = a.nbr[(size_t)k * Nfp + f];
   const int kP = lin / Nfp, fP = lin % Nfp;
@@ -843,7 +929,7 @@ __device__ __forceinline__ void stage_a_body(const StageArgs& a, int k0, double*
   static_assert(!GAUSS || EXT, "Gauss collocation is an EXT mode");
   const int flags = EXT ? a.flags : (a.flags & ~kExtFlags);
   const bool aa = flags & F_AXIS_ALIGNED;
-  Gas<double> g{a.gamma, a.gm1, 2.0 * a.gm1};
+  Gas<double> g{a.gamma, a.gm1, 2.0 * a.gm1, 0.5 * a.rgm1};
   const double dt_lim = a.scal[S_DT_LIM];
   const double t_now = a.scal[S_T];
 
@@ -1483,21 +1569,31 @@ __device__ __forceinline__ void stage_a_body(const StageArgs& a, int k0, double*
         const bool xs = side < 2;
         const double Sxx = (xs ? G[1] : G[2]) * Sv, Sxy = (xs ? G[3] : G[4]) * Sv;
         double* out = base + C::O_FPT + 8 * r;
+        if (aa) {  // the face's own axis only; its other half is 0 and is not read
+          const double Sa = xs ? Sxx : Sxy;
+          double F[4];
+          fS_axis(g, base + C::O_PF + 6 * f, base + C::O_PRIM + 6 * j, xs ? 0 : 1, F);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) out[(xs ? 0 : 4) + c] = Sa * F[c];
+          continue;
+        }
         double Fx[4], Fy[4];
         fS_fast(g, base + C::O_PF + 6 * f, base + C::O_PRIM + 6 * j, Fx, Fy);
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          out[c] = (aa && !xs) ? 0.0 : Sxx * Fx[c];
-          out[4 + c] = (aa && xs) ? 0.0 : Sxy * Fy[c];
+          out[c] = Sxx * Fx[c];
+          out[4 + c] = Sxy * Fy[c];
         }
       }
     }
     __syncthreads();
     if (GAUSS) {
       // face rows of QF1: the pair terms of each face node in the nnz order (j ascending)
-      for (int w = tid; w < Ke * Nfp * 8; w += bs) {
-        int e = w / (Nfp * 8), r = w % (Nfp * 8);
-        int f = r / 8, c = r % 8;
+      // (of axis-aligned elements the face's own axis only)
+      const int nc = aa ? 4 : 8;
+      for (int w = tid; w < Ke * Nfp * nc; w += bs) {
+        int e = w / (Nfp * nc), r = w % (Nfp * nc);
+        int f = r / nc, c = r % nc + (aa && f >= 2 * n ? 4 : 0);
         double* base = sm + e * PE;
         const double* T = base + C::O_FPT + 8 * n * f;
         double q = 0.0;
@@ -1543,7 +1639,8 @@ __device__ __forceinline__ void stage_a_body(const StageArgs& a, int k0, double*
           const int f = fl[t];
           const double* T = base + C::O_FPT + 8 * (n * f + pos[t]);
 #pragma unroll
-          for (int c = 0; c < 8; ++c) Q[c] = Q[c] - T[c];
+          for (int c = 0; c < 8; ++c)
+            if (!aa || (c < 4) == (t < 2)) Q[c] = Q[c] - T[c];
           const double ell = (t % 2 == 0) ? op.ellm[pos[t]] : op.ellp[pos[t]];
           if (limited) {
             const double th = base[C::O_TH + f];
@@ -1558,10 +1655,11 @@ __device__ __forceinline__ void stage_a_body(const StageArgs& a, int k0, double*
         for (int c = 0; c < 8; ++c) {
           double av = rw * Q[c], bv = 0.0;
 #pragma unroll
-          for (int t = 0; t < 4; ++t) {
-            av = av + mf[t] * base[C::O_QFF + 8 * fl[t] + c];
-            bv = bv + mf[t] * base[C::O_BFH + 8 * fl[t] + c];
-          }
+          for (int t = 0; t < 4; ++t)
+            if (!aa || (c < 4) == (t < 2)) {
+              av = av + mf[t] * base[C::O_QFF + 8 * fl[t] + c];
+              bv = bv + mf[t] * base[C::O_BFH + 8 * fl[t] + c];
+            }
           R[c] = (-(av + bv)) * rJ;
         }
       }
