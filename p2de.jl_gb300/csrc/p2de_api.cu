@@ -616,7 +616,7 @@ int p2de_initialize_DG(const p2de_param* prm, const p2de_mesh* mesh, int device,
   s->flux = flags_for(s, 2, false, false) & F_FLUX;
   if (s->flux) {  // its own shared-memory layout
     const FluxShape shape = flux_shape(s->N1D, s->K, s->geo.elems_per_block_flux,
-                                       flags_for(s, 2, false, false) & kExtFlags);
+                                       flags_for(s, 2, false, false) & kExtFlags, s->mixed);
     s->geo.elems_per_block = shape.epb;
     s->geo.elems_per_block_max = s->geo.elems_per_block_max_flux;
     s->base.threads = shape.threads;

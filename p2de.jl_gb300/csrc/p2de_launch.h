@@ -31,16 +31,21 @@ struct StageGeometry {
 //    480x120 N=3 611 and 645. The EXT modes (their time is in the bounds) keep the lines.
 //  * 64 threads otherwise: the lines fill them at the default elements per block, and 128 leave
 //    half the block at that phase's barrier (DMR 480x120 N=3 776 and 656 us, KH 192x192 N=5
-//    1659 and 1376); 128 where a grid is under ten blocks an SM and the shorter phases count.
+//    1659 and 1376); 128 where a grid is under ten blocks an SM and the shorter phases count,
+//    and at N = 2, whose 10 elements fill 128 with nodes (240x120: 220 and 190 us). With FP32
+//    pairs (acc64) the node phases weigh more: N = 5 takes 6 elements and 128 threads (192x192:
+//    841 us against 941 with 5 and 64), N = 4 takes 5 elements (460 against 520 with 6).
 struct FluxShape {
   bool split;
   int epb, threads;
 };
-inline FluxShape flux_shape(int n1d, int K, int epb_lines, bool ext) {
+inline FluxShape flux_shape(int n1d, int K, int epb_lines, bool ext, bool acc64) {
   const int64_t nodes = (int64_t)K * n1d * n1d;
   if (!ext && nodes < (n1d >= 5 ? 110000 : 65536))
     return {true, n1d == 2 ? 8 : n1d == 3 || n1d == 5 ? 3 : 2, 128};
-  return {false, epb_lines, (K + epb_lines - 1) / epb_lines < 10 * 152 ? 128 : 64};
+  if (acc64 && n1d >= 5) epb_lines = n1d == 5 ? 5 : 6;
+  const bool wide = n1d == 3 || (acc64 && n1d == 6) || (K + epb_lines - 1) / epb_lines < 10 * 152;
+  return {false, epb_lines, wide ? 128 : 64};
 }
 
 template <int N1D>
