@@ -85,6 +85,12 @@ struct LineArgs {
 // a finished time loop turns every later launch of the step into a no-op
 __device__ __forceinline__ bool done(const LineArgs& a) { return a.ts[TS_DONE] != 0.0; }
 
+// the limiter's TimeParam dt: the one before the CFL at stage 1 and the given one of a lone RHS,
+// the step's dt at stages 2 and 3
+__device__ __forceinline__ double limiter_dt(const LineArgs& a) {
+  return __longlong_as_double((long long)a.dtkey[(a.flags & LF_UPDATE) && a.nstage > 1 ? 0 : 1]);
+}
+
 // ---- point functions (compressible_Navier_Stokes.jl; four slots, y momentum 0) ----------
 __device__ double pfun4(double gamma, const double* U) {
   return (gamma - 1.0) * (U[3] - div_rn(0.5 * (U[1] * U[1]), U[0]));
@@ -235,7 +241,18 @@ __device__ void Bx(const LineArgs& a, int k, int f, double& b0, double& b1) {
   b0 = g[1] * Br + g[2] * Bs;
   b1 = g[3] * Br + g[4] * Bs;
 }
+__device__ __forceinline__ bool is_zero(double x) { return (__double_as_longlong(x) << 1) == 0; }
+__device__ __forceinline__ bool mid_range(double x) {  // |x| in [2^-500, 2^500)
+  return (unsigned)((__double2hiint(x) & 0x7ff00000) - (523 << 20)) < (1000u << 20);
+}
+// x / n for the components x of a vector of norm n: +-1 exactly along an axis
+__device__ __forceinline__ double unit(double x, double n) {
+  const long long b = __double_as_longlong(x);
+  if (((b ^ __double_as_longlong(n)) << 1) == 0 && mid_range(x)) return b < 0 ? -1.0 : 1.0;
+  return div_rn(x, n);
+}
 __device__ double norm2(double x, double y) {
+  if (is_zero(y) && mid_range(x)) return fabs(x);  // sqrt(x^2) = |x| exactly
   const double m = fmax(fabs(x), fabs(y));
   if (m == 0.0 || isinf(m) || isnan(m)) return m;
   return sqrt_rn(x * x + y * y);
@@ -283,15 +300,11 @@ __device__ void smoothness(const LineArgs& a, const double (*U)[4], double& blen
 // stage begin. dtkey[0]: the step's dt (lowered by the stage-1 CFL), dtkey[1]: the stage's
 // TimeParam dt, which the limiter reads (at stage 1 the dt before the CFL, rhs.jl:41-55 with
 // SSPRK33.jl:30-37). mode 0 (a lone RHS): (dt, dt_lim) from the host, phi reset as given;
-// mode 1 (stages 2, 3 of a step): dtkey[1] = dtkey[0]; mode 2 (stage 1 of a step): from the
+// mode 2 (stage 1 of a step; stages 2 and 3 take dtkey[0], limiter_dt): from the
 // device time t, the loop's end test (SSPRK33.jl:29), dt = min(CFL dt0, T - t) for both,
 // the stage minima reset, and the initial min of phi reset when t == t0 (subcell.jl:31-34).
 __global__ void k_line_begin(LineArgs a, int mode, double dt, double dt_lim, int phi) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  if (mode == 1) {
-    a.dtkey[1] = a.dtkey[0];
-    return;
-  }
   if (mode == 2) {
     const double t = a.ts[TS_T];
     if (!(t < a.T)) {
@@ -525,7 +538,7 @@ __global__ void k_line_low(LineArgs a) {
     const int i = j + 1;
     const double Sr0 = 0.5 * (-0.5 - 0.5), Ss0 = 0.0;
     const double S0 = g[1] * Sr0 + g[2] * Ss0, S1 = g[3] * Sr0 + g[4] * Ss0;
-    const double nn = norm2(S0, S1), n1 = div_rn(S0, nn), n2 = div_rn(S1, nn);
+    const double nn = norm2(S0, S1), n1 = unit(S0, nn), n2 = unit(S1, nn);
     const double ws = jmax(wavespeed4(a.gamma, U[i], n1, n2), wavespeed4(a.gamma, U[j], -n1, -n2));
     const double lij = nn * ws;
     lamR[j] = lij;
@@ -549,8 +562,8 @@ __global__ void k_line_low(LineArgs a) {
     Bx(a, k, f, b0, b1);
     Bx(a, kP, iP, bP0, bP1);
     const double nn = norm2(b0, b1), nnP = norm2(bP0, bP1);
-    wsf[f] = wavespeed4(a.gamma, Uf, div_rn(b0, nn), div_rn(b1, nn));
-    const double wsP = wavespeed4(a.gamma, UfP, div_rn(bP0, nnP), div_rn(bP1, nnP));
+    wsf[f] = wavespeed4(a.gamma, Uf, unit(b0, nn), unit(b1, nn));
+    const double wsP = wavespeed4(a.gamma, UfP, unit(bP0, nnP), unit(bP1, nnP));
     const int8_t bc = a.bc[fk];
     if (bc == BC_INFLOW) {
       const double* I = a.Ival + 3 * (size_t)a.bcidx[fk];
@@ -642,7 +655,7 @@ __global__ void k_line_low_team(LineArgs a) {
     const int j = lane, i = j + 1;
     const double Sr0 = 0.5 * (-0.5 - 0.5), Ss0 = 0.0;
     const double S0 = g[1] * Sr0 + g[2] * Ss0, S1 = g[3] * Sr0 + g[4] * Ss0;
-    const double nn = norm2(S0, S1), n1 = div_rn(S0, nn), n2 = div_rn(S1, nn);
+    const double nn = norm2(S0, S1), n1 = unit(S0, nn), n2 = unit(S1, nn);
     const double ws = jmax(wavespeed4(a.gamma, U[i], n1, n2), wavespeed4(a.gamma, U[j], -n1, -n2));
     const double lij = nn * ws;
     lamR[j] = lij;
@@ -662,8 +675,8 @@ __global__ void k_line_low_team(LineArgs a) {
     Bx(a, k, f, b0, b1);
     Bx(a, kP, iP, bP0, bP1);
     const double nn = norm2(b0, b1), nnP = norm2(bP0, bP1);
-    wsf[f] = wavespeed4(a.gamma, Uf, div_rn(b0, nn), div_rn(b1, nn));
-    const double wsP = wavespeed4(a.gamma, UfP, div_rn(bP0, nnP), div_rn(bP1, nnP));
+    wsf[f] = wavespeed4(a.gamma, Uf, unit(b0, nn), unit(b1, nn));
+    const double wsP = wavespeed4(a.gamma, UfP, unit(bP0, nnP), unit(bP1, nnP));
     const int8_t bc = a.bc[fk];
     if (bc == BC_INFLOW) {
       const double* I = a.Ival + 3 * (size_t)a.bcidx[fk];
@@ -786,7 +799,7 @@ __global__ void k_line_high(LineArgs a) {
   const LineOps& o = *a.ops;
   const double* g = a.geom + 5 * (size_t)k;
   const double J = g[0];
-  const double dt = __longlong_as_double((long long)a.dtkey[1]);  // the limiter's TimeParam dt
+  const double dt = limiter_dt(a);
   double U[MQ][4], ut[MH][4], QF[MH][4];
   for (int i = 0; i < n; ++i) {
     ld4(a.Uq + 4 * ((size_t)n * k + i), U[i]);
@@ -806,8 +819,8 @@ __global__ void k_line_high(LineArgs a) {
     Bx(a, k, f, b0, b1);
     Bx(a, kP, iP, c0, c1);
     const double nn = norm2(b0, b1), nnP = norm2(c0, c1);
-    const double lam = wavespeed4(a.gamma, ut[n + f], div_rn(b0, nn), div_rn(b1, nn));
-    const double lamP = wavespeed4(a.gamma, uP[f], div_rn(c0, nnP), div_rn(c1, nnP));
+    const double lam = wavespeed4(a.gamma, ut[n + f], unit(b0, nn), unit(b1, nn));
+    const double lamP = wavespeed4(a.gamma, uP[f], unit(c0, nnP), unit(c1, nnP));
     LFc[f] = 0.5 * nn * jmax(lam, lamP);
     const int8_t bc = a.bc[fk];
     if (bc == BC_INFLOW || bc == BC_OUTFLOW) {
@@ -1079,7 +1092,7 @@ __global__ void k_line_high_team(LineArgs a) {
   double(*rH)[4] = srH[e];
   double(*rL)[4] = srL[e];
   const double J = live ? a.geom[5 * (size_t)k] : 1.0;
-  const double dt = __longlong_as_double((long long)a.dtkey[1]);  // the limiter's TimeParam dt
+  const double dt = limiter_dt(a);
   if (live) {
     if (lane < n) {
       ld4(a.Uq + 4 * ((size_t)n * k + lane), U[lane]);
@@ -1100,8 +1113,8 @@ __global__ void k_line_high_team(LineArgs a) {
     Bx(a, k, f, b0, b1);
     Bx(a, kP, iP, c0, c1);
     const double nn = norm2(b0, b1), nnP = norm2(c0, c1);
-    const double lam = wavespeed4(a.gamma, ut[n + f], div_rn(b0, nn), div_rn(b1, nn));
-    const double lamP = wavespeed4(a.gamma, uP[f], div_rn(c0, nnP), div_rn(c1, nnP));
+    const double lam = wavespeed4(a.gamma, ut[n + f], unit(b0, nn), unit(b1, nn));
+    const double lamP = wavespeed4(a.gamma, uP[f], unit(c0, nnP), unit(c1, nnP));
     LFc[f] = 0.5 * nn * jmax(lam, lamP);
     const int8_t bc = a.bc[fk];
     if (bc == BC_INFLOW || bc == BC_OUTFLOW) {
@@ -1640,14 +1653,37 @@ cudaError_t launch_stage(LineSolve* L, double t, int nstage, double dt_set, bool
   const int grid = (L->K + kThreads - 1) / kThreads;
   const bool minent = (flags & LF_MINENT) && nstage == 1;
   if (step) {
-    k_line_begin<<<1, 32, 0, L->stream>>>(a, nstage == 1 ? 2 : 1, 0.0, 0.0, minent ? 1 : 0);
+    if (nstage == 1) k_line_begin<<<1, 32, 0, L->stream>>>(a, 2, 0.0, 0.0, minent ? 1 : 0);
   } else {
     // a lone RHS takes the dt it is given, except for the CFL's starting value
     const double dinit = host_jmin(L->prm.CFL * L->prm.dt0, L->prm.T - t);
     const double dkey = (flags & LF_CFL) ? dinit : dt_set;
     k_line_begin<<<1, 32, 0, L->stream>>>(a, 0, dkey, dt_set, (minent && t == L->prm.t0) ? 1 : 0);
   }
-  L->launches += 1;
+  if (!step || nstage == 1) L->launches += 1;
+  // the low-order kernel reads the face projection only with the projected-value flux; without
+  // it, a captured step runs it beside the projection and the pair terms (Shu-Osher K = 64: 26
+  // us beside 31 + 13)
+  const bool beside = L->side && (flags & LF_LOW) && !(flags & LF_LFPROJ);
+  auto launch_low = [&]() {
+    if (line_layout(L) == P2DE_LAYOUT_TEAM) {
+      LINE_LAUNCH(k_line_low_team, (L->K + kTeamE - 1) / kTeamE, a);
+    } else {
+      LINE_LAUNCH(k_line_low, grid, a);
+    }
+    L->launches += 1;
+  };
+  if (beside) {
+    cudaStream_t main = L->stream;
+    cudaError_t e = cudaEventRecord(L->fork, main);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(L->side, L->fork, 0);
+    if (e != cudaSuccess) return e;
+    L->stream = L->side;
+    launch_low();
+    L->stream = main;
+    e = cudaEventRecord(L->join, L->side);
+    if (e != cudaSuccess) return e;
+  }
   if (line_layout(L) == P2DE_LAYOUT_TEAM) {
     switch (L->N1D) {
       case 2: k_line_face_team<2><<<L->K, kFaceTeamThreads, 0, L->stream>>>(a); break;
@@ -1660,14 +1696,7 @@ cudaError_t launch_stage(LineSolve* L, double t, int nstage, double dt_set, bool
     LINE_LAUNCH(k_line_face, (2 * L->K + kThreads - 1) / kThreads, a);
   }
   L->launches += 1;
-  if (flags & LF_LOW) {
-    if (line_layout(L) == P2DE_LAYOUT_TEAM) {
-      LINE_LAUNCH(k_line_low_team, (L->K + kTeamE - 1) / kTeamE, a);
-    } else {
-      LINE_LAUNCH(k_line_low, grid, a);
-    }
-    L->launches += 1;
-  }
+  if ((flags & LF_LOW) && !beside) launch_low();
   if (minent) {  // gated on the device by the begin kernel's t == t0 test
     const long long nodes = (long long)L->K * L->N1D;
     k_line_phimin<<<(int)((nodes + 255) / 256), 256, 0, L->stream>>>(a);
@@ -1676,12 +1705,19 @@ cudaError_t launch_stage(LineSolve* L, double t, int nstage, double dt_set, bool
   if (flags & LF_HIGH) {
     const long long np = (long long)L->K * L->npair;
     k_line_pairs<<<(int)((np + kThreads - 1) / kThreads), kThreads, 0, L->stream>>>(a);
+    if (beside) {
+      const cudaError_t e = cudaStreamWaitEvent(L->stream, L->join, 0);
+      if (e != cudaSuccess) return e;
+    }
     if (line_layout(L) == P2DE_LAYOUT_TEAM) {
       LINE_LAUNCH(k_line_high_team, (L->K + kTeamE - 1) / kTeamE, a);
     } else {
       LINE_LAUNCH(k_line_high, grid, a);
     }
     L->launches += 2;
+  } else if (beside) {
+    const cudaError_t e = cudaStreamWaitEvent(L->stream, L->join, 0);
+    if (e != cudaSuccess) return e;
   }
   if (flags & (LF_SUBCELL | LF_UPDATE)) {
     if (line_layout(L) == P2DE_LAYOUT_TEAM) {
@@ -1985,6 +2021,14 @@ namespace {
 
 // sets the device time, runs `nsteps` loop bodies (one CUDA graph replayed), reads back the
 // time state and the status word once
+void line_drop_branch(LineSolve* L) {
+  if (L->side) cudaStreamDestroy(L->side);
+  if (L->fork) cudaEventDestroy(L->fork);
+  if (L->join) cudaEventDestroy(L->join);
+  L->side = nullptr;
+  L->fork = L->join = nullptr;
+}
+
 int run_steps(LineSolve* L, double* t, int64_t nsteps, double ts_out[TS_N], std::string& err) {
   cudaError_t e = cudaMemcpyAsync(L->ts + TS_T, t, sizeof(double), cudaMemcpyHostToDevice, L->stream);
   if (e == cudaSuccess && nsteps > 1 && !L->graph) {  // capture one body on a private stream
@@ -1993,12 +2037,18 @@ int run_steps(LineSolve* L, double* t, int64_t nsteps, double ts_out[TS_N], std:
     if (e == cudaSuccess) {
       cudaGraph_t g = nullptr;
       const int64_t before = L->launches;
+      // the captured step's second branch (launch_stage); without it the step stays one chain
+      if (cudaStreamCreateWithFlags(&L->side, cudaStreamNonBlocking) != cudaSuccess ||
+          cudaEventCreateWithFlags(&L->fork, cudaEventDisableTiming) != cudaSuccess ||
+          cudaEventCreateWithFlags(&L->join, cudaEventDisableTiming) != cudaSuccess)
+        line_drop_branch(L);
       L->stream = cap;
       e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
       const cudaError_t e1 = e == cudaSuccess ? enqueue_step(L) : e;
       const cudaError_t e2 = e == cudaSuccess ? cudaStreamEndCapture(cap, &g) : e;
       L->stream = user;
       L->launches = before;
+      line_drop_branch(L);
       cudaStreamDestroy(cap);
       e = e1 != cudaSuccess ? e1 : e2;
       if (e == cudaSuccess) e = cudaGraphInstantiate(&L->graph, g, 0);
@@ -2089,7 +2139,7 @@ int line_step_launches(const LineSolve* L) {
   int c = 1;  // k_line_end
   for (int stage = 1; stage <= 3; ++stage) {
     const int f = line_flags(L, stage, true);
-    c += 1 + 1 + ((f & LF_LOW) ? 1 : 0) + ((f & LF_MINENT) && stage == 1 ? 1 : 0) + ((f & LF_HIGH) ? 2 : 0) + 1;
+    c += (stage == 1 ? 1 : 0) + 1 + ((f & LF_LOW) ? 1 : 0) + ((f & LF_MINENT) && stage == 1 ? 1 : 0) + ((f & LF_HIGH) ? 2 : 0) + 1;
   }
   return c;
 }

@@ -36,6 +36,9 @@ struct LineSolve {
   long long* minrec = nullptr;          // min rho, min rhoe per stage (ordered keys)
   double* ts = nullptr;                 // device time state: t, dt, done, steps, phi flag
   cudaGraphExec_t graph = nullptr;      // one SSP-RK3 step, replayed by line_advance
+  // a second branch of the step, only while it is captured
+  cudaStream_t side = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
   int* status = nullptr;
   LineOps* ops = nullptr;
   int64_t launches = 0;
