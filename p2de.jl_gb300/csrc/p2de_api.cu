@@ -816,7 +816,9 @@ int p2de_get_field(p2de_solver* s, int32_t field, int32_t nstage, double* out) {
       const int hl = field == P2DE_FIELD_F_BAR_H ? 0 : 1;
       const int nc = s->kpp ? 1 : 4;  // KPP: the scalar in component 0
       if (s->flux) {
-        // flux form keeps [d][f_H - f_L, f_L][face][c] in units of -g w (p2de_flux.cuh)
+        // flux form keeps [d][f_H - f_L (under F_REF_SEM f_H on interior faces), f_L][face][c] in
+        // units of -g w (p2de_flux.cuh)
+        const bool whole = flags_for(s, 2, false, false) & F_REF_SEM;
         double r[kMaxN1D], w[kMaxN1D], D[kMaxN1D * kMaxN1D];
         gll_rule(s->N, r, w, D);
         std::vector<double> geom(5 * K);
@@ -827,10 +829,12 @@ int p2de_get_field(p2de_solver* s, int32_t field, int32_t nstage, double* out) {
           for (size_t k = 0; k < K; ++k)
             for (size_t f = 0; f < nsf; ++f) {
               const double unit = -(geom[5 * k + (d ? 4 : 1)] * w[d ? f % n : f / (n + 1)]);
+              const size_t t = d ? f / n : f % (n + 1);
+              const bool diff = !whole || t == 0 || t == n;
               for (int c = 0; c < 4; ++c) {
                 const double fL = fb[16 * nsf * k + ((d * 2 + 1) * nsf + f) * 4 + c];
-                const double df = fb[16 * nsf * k + (d * 2 * nsf + f) * 4 + c];
-                out[4 * (f + nsf * (k + K * d)) + c] = unit * (hl == 0 ? fL + df : fL);
+                const double h = fb[16 * nsf * k + (d * 2 * nsf + f) * 4 + c];
+                out[4 * (f + nsf * (k + K * d)) + c] = unit * (hl == 1 ? fL : diff ? fL + h : h);
               }
             }
         return P2DE_OK;

@@ -75,7 +75,10 @@ struct FluxCfg {
   struct Lay {
     static constexpr int O_R = O_W + (EXT ? 14 : 12) * Nq;  // 4 Nq: rhsL; before that CFL sums (0, 1)
     static constexpr int O_PH = O_R + 4 * Nq;               // 4 NF: low-order (then limited) fluxes
-    static constexpr int O_DF = O_PH + 4 * NF;              // 4 NF: high-order minus low-order
+    // 4 NF: high-order minus low-order fluxes; under upper0, where one comparison settles most
+    // interior faces, those hold the high-order flux until a bound asks for the difference
+    // (factor -0 marks those that never did)
+    static constexpr int O_DF = O_PH + 4 * NF;
     static constexpr int O_L = O_DF + 4 * NF;               // NF: factors
     // smoothness factor of the relaxed bounds, 2 flags of the entropy phase, blending factor
     static constexpr int O_X = O_L + NF;
@@ -147,13 +150,13 @@ __device__ __forceinline__ void fS_line(double ig, const PairState& a, const Pai
   *F3 = dmul(f4, un);
 }
 
-// One evaluation of the density bound [Lrho, Urho] (limiter_utils.jl:82-92) with its early
-// out: upper0 (Urho = 0, the Lphi slot of the reference's destructuring), U0 >= Lrho > 0 and
-// P0 >= +0 give U0 + P0 >= Lrho and > 0 = Urho, so the factor max((0 - U0)/P0, 0) is 0.
-__device__ __forceinline__ bool zero_factor(double U0, double P0, double Lrho, bool upper0) {
-  if (!upper0) return false;
-  const long long u = __double_as_longlong(U0), l = __double_as_longlong(Lrho), p = __double_as_longlong(P0);
-  return u > 0 && u < 0x7ff0000000000000LL && l <= u && p >= 0 && p <= 0x7ff0000000000000LL;
+// Whether a node's density factor is 0 for P0 = s dF0 >= +0 under upper0 (Urho = 0, the Lphi
+// slot of the reference's destructuring): U0 >= Lrho > 0 gives U0 + P0 >= Lrho and > 0 = Urho,
+// so the factor max((0 - U0)/P0, 0) is 0.
+__device__ __forceinline__ bool zero_factor(double U0, double s, double Lrho) {
+  const long long u = __double_as_longlong(U0), l = __double_as_longlong(Lrho);
+  return u > 0 && u < 0x7ff0000000000000LL && l <= u &&
+         (__double_as_longlong(s) & 0x7ff0000000000000LL) != 0x7ff0000000000000LL;
 }
 
 // rhoe_quadratic_solve (limiter_utils.jl:108-146) for P = s dF (s the node's 4 dt cx): the
@@ -182,6 +185,13 @@ __device__ __forceinline__ double rhoe_root(const double* U, const double* dF, d
       l = r2;
   }
   return l;
+}
+
+// zeta rhoe_ufun(uL) and c of the quadratics (limiter_utils.jl:141-146)
+__device__ __forceinline__ void energy_bound(const double* uL, double zeta, double& Lrhoe, double& c) {
+  const double ke2 = dfma(uL[1], uL[1], dmul(uL[2], uL[2]));
+  Lrhoe = dmul(zeta, dfma(-0.5, dmul(ke2, rcp(uL[0])), uL[3]));
+  c = dfma(uL[0], dsub(uL[3], Lrhoe), dmul(-0.5, ke2));
 }
 
 // phi = rhoe rho^-gamma (s_modified_ufun) of U + l P, explicitly rounded
@@ -551,7 +561,7 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const int f = ln.comp(q) * NF + ln.f0 + ln.fs * t;
-          ln.DF[f] = dsub(acc[q][t], ln.PH[f]);
+          ln.DF[f] = upper0 ? acc[q][t] : dsub(acc[q][t], ln.PH[f]);
         }
     }
     __syncthreads();
@@ -640,7 +650,7 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
         }
       }
 #pragma unroll
-      for (int t = 1; t < n; ++t) DF[ln.fs * t] = dsub(acc[t], PH[ln.fs * t]);
+      for (int t = 1; t < n; ++t) DF[ln.fs * t] = upper0 ? acc[t] : dsub(acc[t], PH[ln.fs * t]);
     }
     __syncthreads();
   }
@@ -687,12 +697,8 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
       a.rhoL[(size_t)k * Nq + m] = uL[0];
       continue;
     }
-    const double ke2 = dfma(uL[1], uL[1], dmul(uL[2], uL[2]));
-    // zeta rhoe_ufun(uL)
-    const double Lrhoe = dmul(a.zeta, dfma(-0.5, dmul(ke2, rcp(uL[0])), uL[3]));
-    W[C::W_LRHOE * Nq] = Lrhoe;
-    // c of the quadratics (limiter_utils.jl:141-146)
-    W[C::W_QC * Nq] = dfma(uL[0], dsub(uL[3], Lrhoe), dmul(-0.5, ke2));
+    // the internal-energy bound; under upper0 few faces ask for it, and the list forms it
+    if (!upper0) energy_bound(uL, a.zeta, W[C::W_LRHOE * Nq], W[C::W_QC * Nq]);
     // global node index of stencil member t of low_order_stencil (limiter_utils.jl:222-231):
     // r-neighbours, then s-neighbours, across a face through mapP
     auto stencil = [&](int t) -> size_t {
@@ -744,10 +750,11 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
   if (low_only) return;
   __syncthreads();
 
-  // ---- f_bar for p2de_get_field (after p2de_rhs, and the last stage of a step): dF and phi_L
-  //      per element [d][dF, phi_L][face][c]; the debug fields of p2de_rhs
-  const bool dbg = flags & F_WRITE_DEBUG;
-  if (dbg || ((flags & F_UPDATE) && a.nstage == 3)) {
+  // ---- f_bar for p2de_get_field (after p2de_rhs, and the last stage of a step): per element
+  //      [d][DF, phi_L][face][c], DF as O_DF has it here (under upper0 phi_H on interior faces);
+  //      the debug fields of p2de_rhs
+  const bool dbg = flags & F_WRITE_DEBUG, keep_fbar = dbg || ((flags & F_UPDATE) && a.nstage == 3);
+  if (keep_fbar) {
     for (int w = tid; w < Ke * 16 * NSF; w += bs) {
       const int e = w / (16 * NSF), r = w % (16 * NSF);
       const int dh = r / (4 * NSF), f = (dh >> 1) * NSF + (r / 4) % NSF, c = r % 4;
@@ -764,7 +771,10 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
       const double* dy = py + (Y::O_DF - Y::O_PH);
       const double cx = base[C::O_C + ir], cy = base[C::O_C + n + is];
       const double lx = cx * (px[1] - px[0]), ly = cy * (py[n] - py[0]);
-      const double hx = cx * ((px[1] + dx[1]) - (px[0] + dx[0])), hy = cy * ((py[n] + dy[n]) - (py[0] + dy[0]));
+      // phi_H at the node's four faces
+      const double x0 = !upper0 || ir == 0 ? px[0] + dx[0] : dx[0], x1 = !upper0 || ir == n - 1 ? px[1] + dx[1] : dx[1];
+      const double y0 = !upper0 || is == 0 ? py[0] + dy[0] : dy[0], y1 = !upper0 || is == n - 1 ? py[n] + dy[n] : dy[n];
+      const double hx = cx * (x1 - x0), hy = cy * (y1 - y0);
       const size_t g = ((size_t)k0 * Nq) * 8 + (w / 4) * 8 + c;
       a.rhsxyL[g] = lx;
       a.rhsxyL[g + 4] = ly;
@@ -774,6 +784,8 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
       a.rhsH[(size_t)k0 * Nq * 4 + w] = hx + hy;
     }
   }
+
+  if (keep_fbar && upper0) __syncthreads();  // the bounds turn DF into differences in place
 
   // ---- bounds (subcell_bound_limiter!(::Dim2), subcell.jl:288-345). A face's factor is the
   //      min over its one or two nodes: the lower node with P = s dF, the upper with -s dF.
@@ -808,19 +820,31 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
     int d, t, l;
     const int f = face_of(r, d, t, l);
     double* base = sm + e * PE;
-    const double* DF = base + Y::O_DF + f;
+    double* DF = base + Y::O_DF + f;
     const double blend = (flags & F_SHOCK) ? base[Y::O_X + 3] : 1.0;
     double L = blend;
+    double* PHf = base + Y::O_PH + f;
+    const bool inner = r < NI;
+    // the sign of P0 = +-s dF0 settles the bound of one of an interior face's two nodes under
+    // upper0; dF0 = phi_H0 - phi_L0 is negative where its terms compare so
     bool zero = false;
+    if (upper0) {
+      const long long hb = __double_as_longlong(DF[0]), lb = inner ? __double_as_longlong(PHf[0]) : 0;
+      const bool finite = (hb & 0x7ff0000000000000LL) != 0x7ff0000000000000LL &&
+                          (lb & 0x7ff0000000000000LL) != 0x7ff0000000000000LL;
+      const bool neg = inner ? order_key(DF[0]) < order_key(PHf[0]) : hb < 0;
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int m = node_of(d, t, l, h);
-      if (m < 0) continue;
-      // the sign of P0 = +-s dF0 settles the bound of one of the two nodes under upper0
-      const double s = base[C::O_C + 2 * n + d * n + t - 1 + h];
-      const long long sb = __double_as_longlong(s) ^ __double_as_longlong(DF[0]) ^ (h ? (long long)0x8000000000000000ULL : 0LL);
-      const double P0s = __longlong_as_double((sb & (long long)0x8000000000000000ULL) | (__double_as_longlong(DF[0]) & 0x7fffffffffffffffLL));
-      zero = zero || zero_factor(base[C::O_W + C::W_UL * Nq + m], P0s, base[C::O_W + C::W_LRHO * Nq + m], upper0);
+      for (int h = 0; h < 2; ++h) {
+        const int m = node_of(d, t, l, h);
+        if (m < 0 || !finite) continue;
+        const double s = base[C::O_C + 2 * n + d * n + t - 1 + h];
+        const bool down = neg != (negative(s) != (h == 1));  // P0 has its sign bit set
+        zero = zero || (!down && zero_factor(base[C::O_W + C::W_UL * Nq + m], s, base[C::O_W + C::W_LRHO * Nq + m]));
+      }
+    }
+    if (upper0 && !zero && inner) {
+#pragma unroll
+      for (int c = 0; c < 4; ++c) DF[c * NF] = dsub(DF[c * NF], PHf[c * NF]);
     }
     if (!zero) {
 #pragma unroll
@@ -835,7 +859,7 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
         L = min_nonneg_bits(L, fmin(lm, 1.0));
       }
     }
-    if (zero) L = 0.0;
+    if (zero) L = -0.0;  // DF still the high-order flux
     base[Y::O_L + f] = L;
     if (is_zero_bits(L)) continue;
     // dF = 0 (most boundary faces): P = 0 leaves the quadratics' factor 1
@@ -864,7 +888,14 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
       double s = base[C::O_C + 2 * n + d * n + t - 1 + h];
       double is = upper0 ? rcp(s) : base[C::O_C + 4 * n + d * n + t - 1 + h];
       if (h) s = -s, is = -is;
-      double lm = rhoe_root(uL, dF, a4, r2a, W[C::W_QC * Nq], W[C::W_LRHOE * Nq], s, is, a.ZEROTOL);
+      double Lrhoe, qc;
+      if (upper0) {
+        energy_bound(uL, a.zeta, Lrhoe, qc);
+      } else {
+        Lrhoe = W[C::W_LRHOE * Nq];
+        qc = W[C::W_QC * Nq];
+      }
+      double lm = rhoe_root(uL, dF, a4, r2a, qc, Lrhoe, s, is, a.ZEROTOL);
       // the second solve of limiting_param_bound_rho_rhoe: Urhoe = Urho_i (the TVD upper
       // density bound) under the reference semantics, else Inf, for which it returns 1.0
       if (upper0 && (flags & F_TVD)) {
@@ -985,11 +1016,13 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
         const double* vp = base + C::O_W + node_of(d, t, l, 1);
         const double* DF = base + Y::O_DF + f;
         const double* PH = base + Y::O_PH + f;
+        const bool raw = negative(base[Y::O_L + f]);
         double sd = 0.0, sl = 0.0;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           const double dv = dsub(vm[c * Nq], vp[c * Nq]);
-          sd = c ? dfma(dv, DF[c * NF], sd) : dmul(dv, DF[0]);
+          const double df = raw ? dsub(DF[c * NF], PH[c * NF]) : DF[c * NF];
+          sd = c ? dfma(dv, df, sd) : dmul(dv, df);
           sl = c ? dfma(dv, PH[c * NF], sl) : dmul(dv, PH[0]);
         }
         const double dvdf = dmul(gw, sd);
@@ -1084,7 +1117,7 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
 #pragma unroll
       for (int c = 0; c < 4; ++c) PH[c * NF] = dfma(L, DF[c * NF], PH[c * NF]);
     }
-    a.Lpre[(size_t)(k0 + e) * NF + f] = L;
+    a.Lpre[(size_t)(k0 + e) * NF + f] = fabs(L);
     // the face's mark for the node phase below (dF is no longer needed)
     base[Y::O_DF + f] = on ? 1.0 : 0.0;
   }
