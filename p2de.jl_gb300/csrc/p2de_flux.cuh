@@ -417,22 +417,39 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
     c[2 * n] = s;
     if (!upper0) c[4 * n] = rcp(s);
   }
-  for (int w = tid; w < Ke * Nq; w += bs) {
+  // SPLIT deals a node's logarithms to other warps (part 1: log rho; part 2: beta, from its own
+  // copy of p, and log beta), each part in whole warps
+  constexpr int parts = SPLIT && !F32 ? 3 : 1;
+  const int n32 = parts == 1 ? Ke * Nq : (Ke * Nq + 31) & ~31;
+  for (int v = tid; v < parts * n32; v += bs) {
+    const int part = v / n32, w = v % n32;
+    if (w >= Ke * Nq) continue;
     const int e = w / Nq, m = w % Nq;
     double* base = sm + e * PE;
     const double2* src = reinterpret_cast<const double2*>(a.Uq + ((size_t)k0 * Nq + w) * 4);
     const double2 v01 = src[0], v23 = src[1];
     const double rho = v01.x, m1 = v01.y, m2 = v23.x, En = v23.y;
+    if (parts == 3 && part == 1) {
+      base[C::O_W + C::W_LR * Nq + m] = log_fast(rho, op);
+      continue;
+    }
     double* U = base + C::O_U + m;
+    double* W = base + C::O_W + m;
+    const double rr = rcp(rho);
+    // p to the bits of the nodal form: log means of nearly equal states amplify its last bit
+    const double p = dmul(a.gm1, dfma(-0.5, dmul(dfma(m1, m1, dmul(m2, m2)), rr), En));
+    if (parts == 3 && part == 2) {
+      const double beta = dmul(rho, rcp(p));
+      W[C::W_BETA * Nq] = beta;
+      W[C::W_LB * Nq] = log_fast<true>(beta, op);
+      continue;
+    }
     U[0] = rho;
     U[Nq] = m1;
     U[2 * Nq] = m2;
     U[3 * Nq] = En;
-    double* W = base + C::O_W + m;
-    const double rr = rcp(rho), hr = half(rr);
+    const double hr = half(rr);
     const double hu = dmul(m1, hr), hv = dmul(m2, hr);
-    // p to the bits of the nodal form: log means of nearly equal states amplify its last bit
-    const double p = dmul(a.gm1, dfma(-0.5, dmul(dfma(m1, m1, dmul(m2, m2)), rr), En));
     // a state the reference would stop on (DomainError from log or sqrt of a negative,
     // flux_differencing.jl:49-50): density or pressure -0, negative or NaN
     if (!positive_bits(rho) || !positive_bits(p)) atomicOr(a.status, ST_NOT_POSITIVE);
@@ -450,12 +467,14 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
       Wf[2 * Nq] = 2.0f * (float)hv;
       Wf[3 * Nq] = rf / (2.0f * (float)p);
     } else {
-      const double beta = dmul(rho, rcp(p));  // 2 beta of the reference
       W[C::W_U * Nq] = twice(hu);
       W[C::W_V * Nq] = twice(hv);
-      W[C::W_BETA * Nq] = beta;
-      W[C::W_LR * Nq] = log_fast(rho, op);
-      W[C::W_LB * Nq] = log_fast<true>(beta, op);  // log of the reference's beta
+      if (parts == 1) {
+        const double beta = dmul(rho, rcp(p));  // 2 beta of the reference
+        W[C::W_BETA * Nq] = beta;
+        W[C::W_LR * Nq] = log_fast(rho, op);
+        W[C::W_LB * Nq] = log_fast<true>(beta, op);  // log of the reference's beta
+      }
     }
   }
   __syncthreads();
@@ -665,6 +684,16 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
     const double* fy = A + c * NF + NSF + ir + n * is;
     return dfma(base[C::O_C + n + is], dsub(fy[n], fy[0]), dmul(base[C::O_C + ir], dsub(fx[1], fx[0])));
   };
+  if constexpr (SPLIT) {  // one component per thread first
+    for (int w = tid; w < Ke * Nq * 4; w += bs) {
+      const int e = w / (Nq * 4), c = w % (Nq * 4) / Nq, m = w % Nq;
+      double* base = sm + e * PE;
+      const double rl = divergence(base, base + Y::O_PH, m, c);
+      base[Y::O_R + c * Nq + m] = rl;
+      base[C::O_W + (C::W_UL + c) * Nq + m] = dfma(dt_lim, rl, base[C::O_U + c * Nq + m]);
+    }
+    __syncthreads();
+  }
   for (int w = tid; w < Ke * Nq; w += bs) {
     const int e = w / Nq, m = w % Nq, k = k0 + e;
     const int ir = m % n, is = m / n;
@@ -673,12 +702,15 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
     double* R = base + Y::O_R + m;
     double* W = base + C::O_W + m;
     if (flags & F_CFL) {
-      double lx = R[0], ly = R[Nq];
+      double lx, ly;
       if constexpr (SPLIT) {
         const double* wx = base + Y::O_SW + (n + 1) * is + ir;
         const double* wy = base + Y::O_SW + NSF + ir + n * is;
         lx = dadd(wx[0], wx[1]);
         ly = dadd(wy[0], wy[n]);
+      } else {
+        lx = R[0];
+        ly = R[Nq];
       }
       const double lam = dfma(fabs(base[C::O_C + n + is]), ly, dmul(fabs(base[C::O_C + ir]), lx));
       const double d = dmul(a.CFL * 0.5, rcp(lam));
@@ -688,10 +720,14 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
     double uL[4];
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-      const double rl = divergence(base, base + Y::O_PH, m, c);
-      R[c * Nq] = rl;
-      uL[c] = dfma(dt_lim, rl, U[c * Nq]);
-      W[(C::W_UL + c) * Nq] = uL[c];
+      if constexpr (SPLIT) {
+        uL[c] = W[(C::W_UL + c) * Nq];
+      } else {
+        const double rl = divergence(base, base + Y::O_PH, m, c);
+        R[c * Nq] = rl;
+        uL[c] = dfma(dt_lim, rl, U[c * Nq]);
+        W[(C::W_UL + c) * Nq] = uL[c];
+      }
     }
     if (low_only) {  // the low-order densities for the TVD bounds (subcell.jl:112-125)
       a.rhoL[(size_t)k * Nq + m] = uL[0];
