@@ -25,11 +25,9 @@ namespace {
 
 constexpr size_t kScratchDoubles = (size_t)P2DE_NOALLOC_SCRATCH_BYTES / sizeof(double);
 
-// Scratch shared by every call on a device, kept until the process exits. Calls that
+// The scratch is shared by every call on a device and kept until the process exits. Calls that
 // overlap on the GPU (two streams, or a call issued before the previous one finished)
 // race on it.
-static __device__ __align__(256) double g_noalloc_scratch[kScratchDoubles];
-
 // header slots of the scratch, in doubles
 constexpr size_t H_SCAL = 0;         // S_NSCAL doubles
 constexpr size_t H_DTMIN = 8;        // 1 unsigned long long
@@ -40,6 +38,11 @@ constexpr size_t H_COUNTERS = 24;    // 8 unsigned long long
 constexpr size_t H_TABLE = 64;       // OpTable
 constexpr size_t kTableDoubles = (sizeof(OpTable) + 255) / 256 * 256 / sizeof(double);
 constexpr size_t H_DATA = H_TABLE + kTableDoubles;
+// doubles of solve data a call may use: the published budget less the header and the table's
+// first size, so that the largest accepted K does not change as the table grows (the array
+// holds the growth on top)
+constexpr size_t kDataDoubles = kScratchDoubles - H_TABLE - 2976;
+static __device__ __align__(256) double g_noalloc_scratch[H_DATA + kDataDoubles];
 
 struct DeviceState {
   bool ready = false;
@@ -107,7 +110,7 @@ cudaError_t launch_b(int n1d, const StageArgs& a, cudaStream_t st) {
 
 extern "C" int p2de_noalloc_max_elements(int32_t N, int64_t* K_max) {
   if (N < 1 || N > 5 || !K_max) return P2DE_ERR_INVALID_ARGUMENT;
-  *K_max = (int64_t)((kScratchDoubles - H_DATA) / data_doubles_per_elem(N + 1));
+  *K_max = (int64_t)(kDataDoubles / data_doubles_per_elem(N + 1));
   return P2DE_OK;
 }
 
@@ -123,7 +126,7 @@ extern "C" int p2de_rhs_noalloc(const p2de_param* prm, const p2de_device_mesh* m
     return P2DE_ERR_UNSUPPORTED;
   const int n1d = prm->N + 1;
   const size_t K = (size_t)prm->K;
-  if (H_DATA + K * data_doubles_per_elem(n1d) > kScratchDoubles) return P2DE_ERR_BUDGET;
+  if (K * data_doubles_per_elem(n1d) > kDataDoubles) return P2DE_ERR_BUDGET;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return P2DE_ERR_NO_DEVICE;
   cudaStream_t st = (cudaStream_t)stream;
