@@ -1042,7 +1042,19 @@ int p2de_ssp33(p2de_solver* s, double* t_out, int64_t* steps_out, double* dt_las
   CK(cudaSetDevice(s->device));
   double t = s->prm.t0;
   int64_t total = 0;
-  const int rc = p2de_ssp33_advance(s, INT64_MAX, &t, &total);
+  int rc = P2DE_OK;
+  if (s->line) {
+    // a Line step does not look at the status word (a failed 2D step ends the solve on the
+    // device), so the host does, every 64 steps
+    for (;;) {
+      int64_t done = 0;
+      rc = p2de_ssp33_advance(s, 64, &t, &done);
+      total += done;
+      if (rc != P2DE_OK || done < 64 || !(t < s->prm.T)) break;
+    }
+  } else {
+    rc = p2de_ssp33_advance(s, INT64_MAX, &t, &total);
+  }
   if (t_out) *t_out = t;
   if (steps_out) *steps_out = total;
   if (s->line) {
