@@ -44,10 +44,10 @@ METRIC = "DOF-stage updates/s, 2D Euler N=3; served solves/s + p99 vs plain, sam
 UNIT = "DOF-stage updates/s"
 
 # stage kernel A on this workload from one ncu capture
-# (profiles/k_stage_a_dmr480x120_n3_fp64.md): DRAM traffic per launch
+# (profiles/k_flux_a_dmr480x120_n3.md): DRAM traffic per launch
 # (dram__bytes_read.sum + dram__bytes_write.sum) and the FP64 pipe's busy fraction
-KERNEL_A_TRAFFIC_BYTES = 147.9e6
-KERNEL_A_FP64_PIPE_BUSY = 0.825
+KERNEL_A_TRAFFIC_BYTES = 49.3e6
+KERNEL_A_FP64_PIPE_BUSY = 0.835
 
 
 def fma_probe_library():
@@ -721,7 +721,9 @@ def main():
     solver._check(lib.p2de_profile_steps(solver.handle, prof_steps, byref(t), kms))
     solver._check(lib.p2de_read_counters(solver.handle, cnt, 1))
     quad_per_launch = cnt[0] / (3 * prof_steps)
-    flops_a = roofline.stage_a_flops(param.N, desc.K, quad_per_launch)
+    # the workload runs in flux form but for FP32 accumulation and Gauss nodes
+    flux = args.precision != "mixed" and args.basis == "lobatto"
+    flops_a = (roofline.flux_form_flops if flux else roofline.stage_a_flops)(param.N, desc.K, quad_per_launch)
     peak = c_double()
     probe = fma_probe_library()
     rc = probe.p2de_probe_fma_peak(local, 1, byref(peak))
@@ -835,7 +837,7 @@ def main():
             "clocks": clocks,
             "roofline": {
                 "bound": "fp64",
-                "kernel": "k_stage_a (low-order RHS, high-order RHS, limiter bounds)",
+                "kernel": ("k_flux_a" if flux else "k_stage_a") + " (low-order RHS, high-order RHS, limiter bounds)",
                 "achieved": achieved,
                 "peak": peak.value,
                 "unit": "TFLOP/s",

@@ -296,7 +296,8 @@ int p2de_stage_minima(p2de_solver* s, double out[6]);
 int p2de_profile_steps(p2de_solver* s, int64_t nsteps, double* t, double ms[3]);
 
 /* Work counters since the last reset: out[0] = quadratic internal-energy bound
- * solves evaluated (limiter_utils.jl:108-132); the others are skipped exactly. */
+ * solves evaluated (limiter_utils.jl:108-132), or in flux form the faces whose one or two
+ * solves were; the others are skipped exactly. */
 int p2de_read_counters(p2de_solver* s, uint64_t out[1], int32_t reset);
 
 /* Thread layouts. 2D solves: the layout of the high-order volume phases of stage kernel A
@@ -310,13 +311,15 @@ typedef enum p2de_layout {
   P2DE_LAYOUT_FLAT = 0,           /* flat loops over (element, pair) and (element, node) */
   P2DE_LAYOUT_LINES_PER_WARP = 1, /* whole 1D lines per warp: a warp computes the pairs of its
                                      lines, synchronizes only itself and gathers its lines'
-                                     nodes (axis-aligned LGL elements; others run flat) */
+                                     nodes (axis-aligned LGL elements; others run flat, and
+                                     solves in flux form have no pair phase to lay out) */
   P2DE_LAYOUT_TEAM = 2            /* Line solves: a team of lanes per element */
 } p2de_layout;
 
 int p2de_set_layout(p2de_solver* s, int32_t layout);
 int p2de_get_layout(p2de_solver* s, int32_t* layout);
-/* Threads per block of stage kernel A: 64 or 128 (the default). Results do not depend on it. */
+/* Threads per block of stage kernel A: 64 or 128 (the default; solves in flux form pick by the
+ * mesh). Results do not depend on it. */
 int p2de_set_threads_per_block(p2de_solver* s, int32_t threads);
 int p2de_get_threads_per_block(p2de_solver* s, int32_t* threads);
 
@@ -398,7 +401,8 @@ int p2de_server_destroy(p2de_server* s);
  * pool allocator (a Julia or serving process with a fixed HBM budget, where one more
  * cudaMalloc fails or breaks the budget), or an application that allocates device memory
  * only at start-up. All scratch (subcell fluxes, blending factors, device scalars,
- * operator table) lives in one static device array of P2DE_NOALLOC_SCRATCH_BYTES that
+ * operator table) lives in one static device array of P2DE_NOALLOC_SCRATCH_BYTES (and
+ * the operator table's growth since that size was set) that
  * every GPU loading this entry point keeps until the process exits; problems needing
  * more are rejected with P2DE_ERR_BUDGET (p2de_noalloc_max_elements gives the limit per
  * degree). The array is shared by all calls and keeps the last call's contents (the

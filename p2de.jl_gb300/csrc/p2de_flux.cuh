@@ -22,7 +22,7 @@
 // wavespeeds, fluxes and high-order sums in registers: neither pair terms nor nodal fluxes
 // nor wavespeeds go through shared memory, and a node's flux and wavespeed along a line are
 // formed by the one thread that uses them. DMR 480x120 N=3 FP64, per stage: kernel A 1103 us
-// in the nodal form, 656 us here; kernel B 123 us there, 49 us here (it no longer blends).
+// in the nodal form, 590 us here; kernel B 123 us there, 42 us here (it no longer blends).
 //
 // Every operation is an explicitly rounded one (dadd, dmul, dfma ...): nothing is left for
 // the compiler to contract, so the batch kernels give a member the bits it has alone.

@@ -22,6 +22,15 @@ NPL = 2n(n-1), high-order pairs NPH = n^2(n-1), subcell faces NSF = n(n+1):
   bound evaluations (P[0], density bound)                       10 * 4 Nq
   quadratic solves evaluated (P vector, a, b, c, roots)         51 each
   combine per face                                               4 NSF
+
+In flux form (csrc/p2de_flux.cuh), with the interior faces NI = 2n(n-1):
+  nodes: primitives and two logs                               15 Nq
+  node fluxes and wavespeeds along both lines                  22 Nq
+  boundary faces: exterior values, flux, dissipation           37 Nfp
+  interior faces: flux and dissipation                         17 NI
+  high-order pairs: flux, suffix and face sums                 42 NPH
+  low-order rhs and update                                     29 Nq
+  faces listed for a solve: energy bounds, quadratics, blend   70 each
 """
 from __future__ import annotations
 
@@ -59,3 +68,16 @@ def stage_bytes(N: int, K: int) -> dict:
     a = K * (32 * Nq + 32 * Nfp + 40 + 8 * 16 * NSF + 8 * 2 * NSF)
     b = K * (8 * 2 * NSF + 8 * 4 * n + 8 * 16 * NSF + 3 * 32 * Nq + 2 * 32 * Nq + 8 * 2 * NSF + 8)
     return {"stage_a": a, "stage_b": b}
+
+
+def flux_form_flops_per_elem(N: int) -> int:
+    n = N + 1
+    return 66 * n * n + 37 * 4 * n + 17 * 2 * n * (n - 1) + 42 * n * n * (n - 1)
+
+
+FLOPS_PER_LISTED_FACE = 70
+
+
+def flux_form_flops(N: int, K: int, listed_faces: float) -> float:
+    """FP64 operations of one launch of stage kernel A in flux form over K elements."""
+    return flux_form_flops_per_elem(N) * K + FLOPS_PER_LISTED_FACE * listed_faces
