@@ -1016,7 +1016,8 @@ int p2de_ssp33_advance(p2de_solver* s, int64_t nsteps, double* t, int64_t* steps
   CK(cudaStreamSynchronize(s->stream));
   double steps0 = sc[S_STEPS];
   CK(cudaMemcpyAsync(s->scal + S_T, t, sizeof(double), cudaMemcpyHostToDevice, s->stream));
-  double now = sc[S_T] = *t, dt = 0.0;
+  // the last step size, where the call goes on from the last one's time (steps_ahead)
+  double dt = steps0 > 0.0 && sc[S_T] == *t ? sc[S_DT] : 0.0, now = sc[S_T] = *t;
   const int per_step = step_launches(s);
   for (int64_t left = nsteps; left > 0;) {
     const int64_t n = steps_ahead(now, s->prm.T, dt, left);

@@ -147,7 +147,8 @@ inline bool flux_form(int flags, int N, double zerotol, bool own_boundaries, boo
 // Steps to launch before looking at the device's time again: enough to reach T at the last
 // step size, so that a run which ends (or fails) earlier than nsteps does not replay the step
 // as no-ops, seven launches each (the 5x5 vortex solve takes 8 steps of the 64 that
-// p2de_ssp33 asked for: 680 us with the other 56 replayed, 210 without).
+// p2de_ssp33 asked for: 680 us with the other 56 replayed, 210 without). dt: the last step of
+// this run, 0 at its start.
 inline int64_t steps_ahead(double t, double T, double dt, int64_t left) {
   const int64_t first = 4, most = 4096;
   if (!(dt > 0.0)) return left < first ? left : first;

@@ -2019,8 +2019,6 @@ int line_rhs(LineSolve* L, double t, double dt, int nstage, double* dt_out, std:
 
 namespace {
 
-// sets the device time, runs `nsteps` loop bodies (one CUDA graph replayed), reads back the
-// time state and the status word once
 void line_drop_branch(LineSolve* L) {
   if (L->side) cudaStreamDestroy(L->side);
   if (L->fork) cudaEventDestroy(L->fork);
@@ -2029,7 +2027,10 @@ void line_drop_branch(LineSolve* L) {
   L->fork = L->join = nullptr;
 }
 
-int run_steps(LineSolve* L, double* t, int64_t nsteps, double ts_out[TS_N], std::string& err) {
+// sets the device time, runs up to `nsteps` loop bodies (one CUDA graph replayed; dt: the last
+// step size or 0, for steps_ahead), reads back the time state between batches and the status
+// word once
+int run_steps(LineSolve* L, double* t, int64_t nsteps, double dt, double ts_out[TS_N], std::string& err) {
   cudaError_t e = cudaMemcpyAsync(L->ts + TS_T, t, sizeof(double), cudaMemcpyHostToDevice, L->stream);
   if (e == cudaSuccess && nsteps > 1 && !L->graph) {  // capture one body on a private stream
     cudaStream_t cap, user = L->stream;
@@ -2056,7 +2057,7 @@ int run_steps(LineSolve* L, double* t, int64_t nsteps, double ts_out[TS_N], std:
     }
   }
   const int per_step = line_step_launches(L);
-  double now = *t, dt = 0.0;
+  double now = *t;
   int64_t left = nsteps;
   do {
     const int64_t n = steps_ahead(now, L->prm.T, dt, left);
@@ -2089,7 +2090,7 @@ int run_steps(LineSolve* L, double* t, int64_t nsteps, double ts_out[TS_N], std:
 int line_step(LineSolve* L, double* t, double* dt_out, std::string& err) {
   double ts[TS_N];
   double tt = *t;
-  const int rc = run_steps(L, &tt, 1, ts, err);
+  const int rc = run_steps(L, &tt, 1, 0.0, ts, err);
   if (rc != P2DE_OK) return rc;
   const bool stepped = ts[TS_DONE] == 0.0;
   if (dt_out) *dt_out = stepped ? ts[TS_DT] : 0.0;
@@ -2106,7 +2107,7 @@ int line_advance(LineSolve* L, int64_t nsteps, double* t, int64_t* steps_done, d
     return P2DE_ERR_CUDA;
   }
   const double steps0 = ts[TS_STEPS];
-  const int rc = run_steps(L, t, nsteps, ts, err);
+  const int rc = run_steps(L, t, nsteps, steps0 > 0.0 && ts[TS_T] == *t ? ts[TS_DT] : 0.0, ts, err);
   if (steps_done) *steps_done = (int64_t)(ts[TS_STEPS] - steps0);
   if (dt_last) *dt_last = ts[TS_DT];
   return rc;
