@@ -187,27 +187,46 @@ static void split_hi_lo(long double v, int bits, double* hi, double* lo) {
   *lo = (double)(v - (long double)h);
 }
 
+// The tables of log_fast and exp_fast, the same for every solve: formed once per process, as
+// the long double functions run in software on Arm (about 130 us of a solver's creation)
+struct FunctionTables {
+  double logtab[kLogTabN][3];
+  double ln2_hi, ln2_lo;
+  double exptab[128][2];
+  double exp_inv, exp_hi, exp_lo;
+  FunctionTables() {
+    for (int i = 0; i < kLogTabN; ++i) {
+      const int j = kLogTabLo + i;
+      logtab[i][0] = 256.0 / j;
+      split_hi_lo(std::log((long double)j / 256.0L), 41, &logtab[i][1], &logtab[i][2]);
+    }
+    split_hi_lo(std::log(2.0L), 42, &ln2_hi, &ln2_lo);
+    for (int j = 0; j < 128; ++j) {
+      const long double v = std::exp2((long double)j / 128.0L);
+      exptab[j][0] = (double)v;
+      exptab[j][1] = (double)(v - (long double)exptab[j][0]);
+    }
+    exp_inv = (double)(128.0L / std::log(2.0L));
+    split_hi_lo(std::log(2.0L) / 128.0L, 35, &exp_hi, &exp_lo);
+  }
+};
+
 template <class Tab>
-static void fill_log_table(Tab* T) {
-  for (int i = 0; i < kLogTabN; ++i) {
-    const int j = kLogTabLo + i;
-    T->logtab[i][0] = 256.0 / j;
-    split_hi_lo(std::log((long double)j / 256.0L), 41, &T->logtab[i][1], &T->logtab[i][2]);
-  }
-  split_hi_lo(std::log(2.0L), 42, &T->ln2_hi, &T->ln2_lo);
-  for (int j = 0; j < 128; ++j) {
-    const long double v = std::exp2((long double)j / 128.0L);
-    T->exptab[j][0] = (double)v;
-    T->exptab[j][1] = (double)(v - (long double)T->exptab[j][0]);
-  }
-  T->exp_inv = (double)(128.0L / std::log(2.0L));
-  split_hi_lo(std::log(2.0L) / 128.0L, 35, &T->exp_hi, &T->exp_lo);
+static void fill_function_tables(Tab* T) {
+  static const FunctionTables t;
+  std::memcpy(T->logtab, t.logtab, sizeof t.logtab);
+  T->ln2_hi = t.ln2_hi;
+  T->ln2_lo = t.ln2_lo;
+  std::memcpy(T->exptab, t.exptab, sizeof t.exptab);
+  T->exp_inv = t.exp_inv;
+  T->exp_hi = t.exp_hi;
+  T->exp_lo = t.exp_lo;
 }
 
 int build_op_table(int N, double zerotol, OpTable* T, int basis) {
   if (N < 1 || N + 1 > kMaxN1D || basis < 0 || basis > 1) return 1;
   std::memset(T, 0, sizeof(OpTable));
-  fill_log_table(T);
+  fill_function_tables(T);
   const int n = N + 1, Nq = n * n;
   T->N1D = n;
   T->Nq = Nq;
@@ -389,7 +408,7 @@ namespace p2de {
 int build_line_ops(int N, double zerotol, LineOps* T, int basis) {
   if (N < 1 || N + 1 > kMaxN1D || basis < 0 || basis > 1) return 1;
   std::memset(T, 0, sizeof(LineOps));
-  fill_log_table(T);
+  fill_function_tables(T);
   const int n = N + 1, Nh = n + 2;
   double r[kMaxN1D], w[kMaxN1D], D[kMaxN1D * kMaxN1D], ellm[kMaxN1D], ellp[kMaxN1D];
   if (basis == 1) {
