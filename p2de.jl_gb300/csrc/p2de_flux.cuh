@@ -296,8 +296,9 @@ struct FluxLine {
     P.U[3] = S[3];
     const double rr = rcp(P.U[0]), hr = half(rr);
     const double hn = dmul(P.U[1], hr), ht = dmul(P.U[2], hr);
-    const double pe = dsub(P.U[3], dfma(P.U[1], hn, dmul(P.U[2], ht)));
-    line_node(P, hn, ht, dmul(a.hgm1, pe), dmul(a.cws, rr));
+    // p as the node phase forms it, so that the two elements at a face form the same flux bits
+    const double p = dmul(a.gm1, dfma(-0.5, dmul(dfma(S[1], S[1], dmul(S[2], S[2])), rr), S[3]));
+    line_node(P, hn, ht, half(p), dmul(a.cws, rr));
     // a boundary face's wavespeed is the own one (its mapP is itself)
     if (code != BC_INTERIOR) P.wh = own.wh;
     off = code == BC_INFLOW || code == BC_OUTFLOW || code == BC_SHOCK;
