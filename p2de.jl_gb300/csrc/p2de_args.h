@@ -78,7 +78,8 @@ struct StageArgs {
   double* BFL;
   double* BFH;
   double* fbar;  // K x (2 dirs x 2 (H, L) x NSF x 4)
-  double* Lpre;  // K x 2 x (Nq+N1D), before symmetrization
+  double* Lpre;  // K x 2 x (Nq+N1D), before symmetrization (nodal form: a set sign bit marks
+                 // a face whose fluxes overflow)
   double* Lfin;  // 3 stages x K x 2 x (Nq+N1D)
   double* scal;  // S_* slots
   unsigned long long* dtmin_bits;

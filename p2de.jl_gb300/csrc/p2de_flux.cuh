@@ -1148,9 +1148,19 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
     const double L = base[Y::O_L + f];
     double* PH = base + Y::O_PH + f;
     const double* DF = base + Y::O_DF + f;
-    const bool on = !is_zero_bits(L) && (r < NI || !(is_zero_bits(DF[0]) && is_zero_bits(DF[NF]) &&
-                                                     is_zero_bits(DF[2 * NF]) && is_zero_bits(DF[3 * NF])));
-    if (on) {
+    bool on = !is_zero_bits(L) && (r < NI || !(is_zero_bits(DF[0]) && is_zero_bits(DF[NF]) &&
+                                               is_zero_bits(DF[2 * NF]) && is_zero_bits(DF[3 * NF])));
+    bool inf = false;  // the face's fluxes overflow: phi + l (phi_H - phi_L) also where l is 0
+#pragma unroll
+    for (int c = 0; c < 4; ++c) inf = inf || may_overflow(DF[c * NF]) || may_overflow(PH[c * NF]);
+    if (inf) {
+#pragma unroll 1
+      for (int c = 0; c < 4; ++c) {
+        const double h = negative(L) ? DF[c * NF] : dadd(PH[c * NF], DF[c * NF]);
+        PH[c * NF] = dfma(fabs(L), dsub(h, PH[c * NF]), PH[c * NF]);
+      }
+      on = true;
+    } else if (on) {
 #pragma unroll
       for (int c = 0; c < 4; ++c) PH[c * NF] = dfma(L, DF[c * NF], PH[c * NF]);
     }

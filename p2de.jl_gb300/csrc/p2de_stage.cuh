@@ -201,6 +201,11 @@ __device__ __forceinline__ bool magnitude_above(double x, double t) {
   return b > __double_as_longlong(t) && b <= 0x7ff0000000000000LL;
 }
 
+// |x| >= 2^1023, infinite or NaN: a difference with it may not be finite
+__device__ __forceinline__ bool may_overflow(double x) {
+  return (__double2hiint(x) & 0x7fffffff) >= 0x7fe00000;
+}
+
 // fluxes(Dim2) (:175-194) with 1/rho given
 __device__ __forceinline__ void fluxes_r(const Gas<double>& g, const double* U, double rr, double* fx, double* fy) {
   double rho = U[0], rhou = U[1], rhov = U[2], E = U[3];
@@ -772,10 +777,11 @@ __device__ __forceinline__ void es_interface_body(const StageArgs& a, long long 
     dvB[c] = __dsub_rn(vB[c], vA[c]);
   }
   const size_t iA = lidx(k, f), iB = lidx(kP, fP);
-  const double LA = solve(a.Lpre[iA], a.Lpre[iB], dvf(k, f, dvA, a.BFH), dvf(k, f, dvA, a.BFL), dpsi);
-  const double LB = solve(a.Lpre[iB], LA, dvf(kP, fP, dvB, a.BFH), dvf(kP, fP, dvB, a.BFL), -dpsi);
-  a.Lpre[iA] = LA;
-  a.Lpre[iB] = LB;
+  const double mA = a.Lpre[iA], mB = a.Lpre[iB];  // with their marks (kernel A, P12)
+  const double LA = solve(fabs(mA), fabs(mB), dvf(k, f, dvA, a.BFH), dvf(k, f, dvA, a.BFL), dpsi);
+  const double LB = solve(fabs(mB), LA, dvf(kP, fP, dvB, a.BFH), dvf(kP, fP, dvB, a.BFL), -dpsi);
+  a.Lpre[iA] = copysign(LA, mA);
+  a.Lpre[iB] = copysign(LB, mB);
 }
 
 template <int N1D>
@@ -2292,14 +2298,21 @@ __device__ __forceinline__ void stage_a_body(const StageArgs& a, int k0, double*
     __syncthreads();
   }
 
-  // ---- P12: L before symmetrization and the subcell fluxes for kernel B
+  // ---- P12: the subcell fluxes and L before symmetrization for kernel B. A face whose fluxes
+  //      overflow (FP32 terms do from 2^128 on) has the sign bit of its L set: kernel B then
+  //      forms the combination also where L is 0, whose 0 x Inf = NaN ends the step.
+  for (int w = tid; w < Ke * C::FBAR; w += bs) {
+    const int e = w / C::FBAR, r = w % C::FBAR;
+    const double v = sm[e * PE + C::O_SCR + r];
+    a.fbar[(size_t)(k0 + e) * C::FBAR + r] = v;
+    if (may_overflow(v))
+      atomicOr(reinterpret_cast<unsigned long long*>(sm + e * PE + C::O_L + r / (8 * NSF) * NSF + r / 4 % NSF),
+               0x8000000000000000ULL);
+  }
+  __syncthreads();
   for (int w = tid; w < Ke * 2 * NSF; w += bs) {
     int e = w / (2 * NSF), r = w % (2 * NSF);
     a.Lpre[(size_t)(k0 + e) * 2 * NSF + r] = sm[e * PE + C::O_L + r];
-  }
-  for (int w = tid; w < Ke * C::FBAR; w += bs) {
-    int e = w / C::FBAR, r = w % C::FBAR;
-    a.fbar[(size_t)(k0 + e) * C::FBAR + r] = sm[e * PE + C::O_SCR + r];
   }
 }
 
@@ -2367,12 +2380,14 @@ __device__ __forceinline__ void stage_b_body(const StageArgs& a, int k0, double*
       }
       double own = a.Lpre[(size_t)k * 2 * NSF + d * NSF + idx];
       double par = a.Lpre[(size_t)kP * 2 * NSF + d * NSF + idxP];
-      sm[e * PE + d * NSF + idx] = fmin(own, par);
+      // the sign is the own fluxes' mark (P12)
+      sm[e * PE + d * NSF + idx] = copysign(fmin(fabs(own), fabs(par)), own);
     }
     __syncthreads();
     // accumulate_f_bar_limited!(::Dim2) (subcell.jl:841-876), one face per thread, the interior
-    // faces of all elements first: a face with factor 0 (under the reference's reading, every
-    // interior one) takes fL without reading fH and without an FP64 instruction
+    // faces of all elements first: a face with factor +0 (under the reference's reading, every
+    // interior one) takes fL without reading fH and without an FP64 instruction; -0 is a face
+    // whose fluxes overflow (P12)
     constexpr int NI = 2 * n * (n - 1);
     for (int w = tid; w < Ke * 2 * NSF; w += bs) {
       const int e = w < Ke * NI ? w / NI : (w - Ke * NI) / (4 * n);
@@ -2395,12 +2410,13 @@ __device__ __forceinline__ void stage_b_body(const StageArgs& a, int k0, double*
       const double2* g = reinterpret_cast<const double2*>(a.fbar + (size_t)(k0 + e) * C::FBAR + (d * 2 * NSF + fi) * 4);
       double2 lo = g[2 * NSF], hi = g[2 * NSF + 1];
       // l fH + (1 - l) fL as fL + l (fH - fL): one rounding fewer, and exactly fL at l = 0
-      if (!is_zero_bits(l)) {
+      if (__double_as_longlong(l) != 0) {
         const double2 h0 = g[0], h1 = g[1];
-        lo.x = fma(l, h0.x - lo.x, lo.x);
-        lo.y = fma(l, h0.y - lo.y, lo.y);
-        hi.x = fma(l, h1.x - hi.x, hi.x);
-        hi.y = fma(l, h1.y - hi.y, hi.y);
+        const double lm = fabs(l);
+        lo.x = fma(lm, h0.x - lo.x, lo.x);
+        lo.y = fma(lm, h0.y - lo.y, lo.y);
+        hi.x = fma(lm, h1.x - hi.x, hi.x);
+        hi.y = fma(lm, h1.y - hi.y, hi.y);
       }
       double2* out = reinterpret_cast<double2*>(base + C::O_FLIM + (d * NSF + fi) * 4);
       out[0] = lo;
@@ -2481,7 +2497,7 @@ __device__ __forceinline__ void stage_b_body(const StageArgs& a, int k0, double*
   if (limited) {
     for (int w = tid; w < Ke * 2 * NSF; w += bs) {
       int e = w / (2 * NSF), r = w % (2 * NSF);
-      a.Lfin[((size_t)s * a.K + k0 + e) * 2 * NSF + r] = sm[e * PE + r];
+      a.Lfin[((size_t)s * a.K + k0 + e) * 2 * NSF + r] = fabs(sm[e * PE + r]);
     }
   }
   if (flags & F_UPDATE) {

@@ -1,0 +1,59 @@
+"""Subcell fluxes that overflow: a limited flux f_L + l (f_H - f_L) with either one infinite or
+NaN is not finite, whatever the factor l (0 x Inf is NaN), so the step ends with an error and
+the right-hand side shows where. FP32 two-point fluxes overflow from 2^128 on."""
+import numpy as np
+import pytest
+
+import p2de
+from p2de import abi, problems
+from p2de import solver as S
+from p2de.types import PositivityAndCellEntropyBound, PositivityAndMinEntropyBound, PositivityBound, TVDBound
+
+from helpers import setup
+
+pytestmark = pytest.mark.gpu
+
+NOT_POSITIVE = 5
+BOUNDS = {"pos": PositivityBound(), "cell": PositivityAndCellEntropyBound(), "tvd": TVDBound(),
+          "min": PositivityAndMinEntropyBound()}
+
+
+def solver_with(problem, N, bound, reference, precision, energy):
+    param, md, bc, desc, U0 = setup(problem, N=N, Kx=6, Ky=4, bound=BOUNDS[bound], precision=precision,
+                                    reference_semantics=reference)
+    U = U0.copy()
+    U[9, 1, 3] = energy
+    g = S.Solver(param, md, desc)
+    g.set_Uq(U)
+    return g
+
+
+@pytest.mark.parametrize("precision,energy", [("fp64", np.inf), ("mixed", 1e60), ("mixed-acc64", 1e60)])
+@pytest.mark.parametrize("reference", [True, False])
+@pytest.mark.parametrize("bound", list(BOUNDS))
+@pytest.mark.parametrize("N", [1, 3])
+def test_overflowed_fluxes_reach_the_right_hand_side(N, bound, reference, precision, energy):
+    g = solver_with(problems.riemann2d, N, bound, reference, precision, energy)
+    S.rhs_bang(None, g, None, p2de.TimeParam(0.0, 1e-6, 2))
+    n, K = N + 1, 24
+    bad = ~np.isfinite(g.get_field(abi.FIELD_F_BAR_H)) | ~np.isfinite(g.get_field(abi.FIELD_F_BAR_L))
+    bad = bad.reshape(2, K, n * (n + 1), 4)
+    fx = bad[0].reshape(K, n, n + 1, 4)  # [line][face]
+    fy = bad[1].reshape(K, n + 1, n, 4)  # [face][line]
+    want = fx[:, :, 1:] | fx[:, :, :-1] | fy[:, 1:] | fy[:, :-1]
+    assert want.any()
+    np.testing.assert_array_equal(~np.isfinite(g.get_field(abi.FIELD_RHSU)).reshape(want.shape), want)
+    L = g.get_field(abi.FIELD_L_LOCAL, 2)
+    assert not np.signbit(L).any() and (L <= 1).all()
+    g.close()
+
+
+@pytest.mark.parametrize("precision", ["mixed", "mixed-acc64"])
+@pytest.mark.parametrize("bound", list(BOUNDS))
+@pytest.mark.parametrize("N", [1, 3])
+def test_a_step_with_overflowed_fluxes_fails(N, bound, precision):
+    g = solver_with(problems.riemann2d, N, bound, True, precision, 1e60)
+    with pytest.raises(abi.P2deError) as ei:
+        S.ssp33_step(g, 0.0)
+    assert ei.value.status == NOT_POSITIVE
+    g.close()
