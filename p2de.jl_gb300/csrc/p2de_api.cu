@@ -1044,17 +1044,14 @@ int p2de_ssp33(p2de_solver* s, double* t_out, int64_t* steps_out, double* dt_las
   double t = s->prm.t0;
   int64_t total = 0;
   int rc = P2DE_OK;
-  if (s->line) {
-    // a Line step does not look at the status word (a failed 2D step ends the solve on the
-    // device), so the host does, every 64 steps
-    for (;;) {
-      int64_t done = 0;
-      rc = p2de_ssp33_advance(s, 64, &t, &done);
-      total += done;
-      if (rc != P2DE_OK || done < 64 || !(t < s->prm.T)) break;
-    }
-  } else {
-    rc = p2de_ssp33_advance(s, INT64_MAX, &t, &total);
+  // 64 steps at a time: where the time step grows, or a step fails, the steps launched ahead do
+  // nothing (steps_ahead takes the rest of the run at the last step size), and a Line step does
+  // not look at the status word, so the host does
+  for (;;) {
+    int64_t done = 0;
+    rc = p2de_ssp33_advance(s, 64, &t, &done);
+    total += done;
+    if (rc != P2DE_OK || done < 64 || !(t < s->prm.T)) break;
   }
   if (t_out) *t_out = t;
   if (steps_out) *steps_out = total;
