@@ -1156,7 +1156,8 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
     if (inf) {
 #pragma unroll 1
       for (int c = 0; c < 4; ++c) {
-        const double h = negative(L) ? DF[c * NF] : dadd(PH[c * NF], DF[c * NF]);
+        // only interior faces keep phi_H in DF (O_DF)
+        const double h = r < NI && negative(L) ? DF[c * NF] : dadd(PH[c * NF], DF[c * NF]);
         PH[c * NF] = dfma(fabs(L), dsub(h, PH[c * NF]), PH[c * NF]);
       }
       on = true;

@@ -1,6 +1,8 @@
 """Subcell fluxes that overflow: a limited flux f_L + l (f_H - f_L) with either one infinite or
 NaN is not finite, whatever the factor l (0 x Inf is NaN), so the step ends with an error and
 the right-hand side shows where. FP32 two-point fluxes overflow from 2^128 on."""
+from dataclasses import replace
+
 import numpy as np
 import pytest
 
@@ -56,4 +58,24 @@ def test_a_step_with_overflowed_fluxes_fails(N, bound, precision):
     with pytest.raises(abi.P2deError) as ei:
         S.ssp33_step(g, 0.0)
     assert ei.value.status == NOT_POSITIVE
+    g.close()
+
+
+@pytest.mark.parametrize("rho", [1.0, 20.0])
+def test_large_boundary_fluxes_with_a_finite_difference_stay_finite(rho):
+    """At an inflow face the low-order flux and the dissipation it has on top of the high-order
+    one reach 2^1023 here; the high-order flux is 0 in the energy, so nothing overflows (the
+    nodal form scales its fluxes in another order and overflows)."""
+    param, md, bc, _, U0 = setup(problems.double_mach_reflection, N=1, Kx=8, Ky=2)
+    geom = md.geom.copy()
+    geom[:, 0] *= 2.0**16  # the right-hand side is the flux over J
+    U = np.zeros_like(U0)
+    U[..., 0] = rho
+    # half the wavespeed times E: 1.06 x 2^1023 and 1.08 x 2^1023
+    U[..., 3] = 2.0**683 * (1.0 if rho == 1.0 else 2.75)
+    g = S.Solver(param, md, S.make_descriptor(param, replace(md, geom=geom), bc))
+    g.set_Uq(U)
+    S.rhs_bang(None, g, None, p2de.TimeParam(0.0, 2.0**-700, 2))
+    assert np.isfinite(g.get_field(abi.FIELD_F_BAR_L)).all() and np.isfinite(g.get_field(abi.FIELD_F_BAR_H)).all()
+    assert np.isfinite(g.get_field(abi.FIELD_RHSU)).all()
     g.close()
