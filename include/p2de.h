@@ -361,7 +361,9 @@ int p2de_batch_memory(p2de_batch* b, size_t* used, size_t* capacity);
 int p2de_batch_launch_count(p2de_batch* b, int64_t* count);
 int p2de_batch_last_error(p2de_batch* b, char* buf, size_t len);
 /* Elements per block of the batch's tasks for degree N (1..5); as for one solve,
- * results do not depend on it. */
+ * results do not depend on it. Until it is set or tuned, members in flux form and others
+ * run at defaults of their own; the getter gives the one of the members present, the flux
+ * form's where both are. */
 int p2de_batch_set_elements_per_block(p2de_batch* b, int32_t N, int32_t epb);
 int p2de_batch_get_elements_per_block(p2de_batch* b, int32_t N, int32_t* epb, int32_t* epb_max);
 /* Thread layout (p2de_layout) of the batch's tasks for degree N; results do not depend on it. */

@@ -333,6 +333,18 @@ int kind_epb(const p2de_batch* b, int n1d, int kind) {
   return b->epb[n1d] > 0 ? b->epb[n1d] : batch_elems_per_block(n1d, kind >= BATCH_FLUX);
 }
 
+// the elements per block that a degree's members run at; 0 members: those that a member would.
+// Members of both forms at their own defaults: the flux form's.
+int degree_epb(const p2de_batch* b, int n1d) {
+  bool nodal = false, flux = false;
+  for (int s = 0; s < b->max_solves; ++s) {
+    const Slot& sl = b->slots[s];
+    if (sl.active && sl.n1d == n1d) (batch_kind(sl.flags) >= BATCH_FLUX ? flux : nodal) = true;
+  }
+  if (!nodal && !flux) nodal = b->precision == P2DE_PRECISION_MIXED;
+  return kind_epb(b, n1d, nodal && !flux ? BATCH_PLAIN : BATCH_FLUX);
+}
+
 // The tasks of one member: elements in runs of the degree's elements per block.
 void member_tasks(const p2de_batch* b, int s, std::vector<BatchTask>& t) {
   const Slot& sl = b->slots[s];
@@ -746,7 +758,7 @@ int p2de_batch_get_layout(p2de_batch* b, int32_t N, int32_t* layout) {
 
 int p2de_batch_get_elements_per_block(p2de_batch* b, int32_t N, int32_t* epb, int32_t* epb_max) {
   if (!b || N < 1 || N + 1 > kMaxN1D) return P2DE_ERR_INVALID_ARGUMENT;
-  if (epb) *epb = kind_epb(b, N + 1, BATCH_FLUX);
+  if (epb) *epb = degree_epb(b, N + 1);
   if (epb_max) *epb_max = batch_elems_per_block_max(N + 1);
   return P2DE_OK;
 }
@@ -799,18 +811,20 @@ int p2de_batch_autotune(p2de_batch* b, int32_t best_epb[5]) {
     bool present = false;
     for (int s = 0; s < b->max_solves; ++s) present |= b->slots[s].active && b->slots[s].n1d == n1d;
     if (!present) continue;
-    const int emax = batch_elems_per_block_max(n1d), edef = batch_elems_per_block(n1d, true);
-    int best = edef, best_layout = b->layout[n1d];
+    const int emax = batch_elems_per_block_max(n1d);
+    int best = 0, best_layout = b->layout[n1d];
     double bms = 1e30;
     for (int lay : {(int)P2DE_LAYOUT_FLAT, (int)P2DE_LAYOUT_LINES_PER_WARP})
-    for (int e : {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, edef}) {
-      if (e > emax) continue;
+    for (int c : {0, 1, 2, 3, 4, 6, 8, 12, 16, 24, 32}) {  // 0: each kind's default
+      if (c > emax) continue;
+      auto epb_of = [&](int kind) { return c > 0 ? c : batch_elems_per_block(n1d, kind >= BATCH_FLUX); };
       // this degree's members by kind, full pass at stage 2
       std::vector<BatchTask> t[BATCH_KINDS], all;
       for (int s = 0; s < b->max_solves; ++s) {
         const Slot& sl = b->slots[s];
         if (!sl.active || sl.n1d != n1d) continue;
-        for (int k0 = 0; k0 < sl.prm.K; k0 += e) t[batch_kind(sl.flags)].push_back(BatchTask{s, k0, n1d, e, lay});
+        const int kind = batch_kind(sl.flags), e = epb_of(kind);
+        for (int k0 = 0; k0 < sl.prm.K; k0 += e) t[kind].push_back(BatchTask{s, k0, n1d, e, lay});
       }
       int grid[BATCH_KINDS] = {}, nt[BATCH_KINDS], off[BATCH_KINDS];
       size_t sm[BATCH_KINDS];
@@ -818,7 +832,7 @@ int p2de_batch_autotune(p2de_batch* b, int32_t best_epb[5]) {
       for (int x = 0; x < BATCH_KINDS; ++x) {
         nt[x] = (int)t[x].size();
         off[x] = (int)all.size();
-        sm[x] = batch_smem_a(n1d, e, x);
+        sm[x] = batch_smem_a(n1d, epb_of(x), x);
         all.insert(all.end(), t[x].begin(), t[x].end());
         if (!nt[x]) continue;
         int bpa = 0;
@@ -846,13 +860,13 @@ int p2de_batch_autotune(p2de_batch* b, int32_t best_epb[5]) {
       }
       if (tot / 3.0 < bms) {
         bms = tot / 3.0;
-        best = e;
+        best = c;
         best_layout = lay;
       }
     }
     b->epb[n1d] = best;
     b->layout[n1d] = best_layout;
-    if (best_epb) best_epb[n1d - 2] = best;
+    if (best_epb) best_epb[n1d - 2] = degree_epb(b, n1d);
   }
   return P2DE_OK;
   };
