@@ -615,8 +615,10 @@ int p2de_initialize_DG(const p2de_param* prm, const p2de_mesh* mesh, int device,
                       own_faces(mesh->mapW, mesh->nW, mesh->mapP) && own_faces(mesh->mapS, mesh->nS, mesh->mapP);
   s->flux = flags_for(s, 2, false, false) & F_FLUX;
   if (s->flux) {  // its own shared-memory layout
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return bail(P2DE_ERR_CUDA);
     const FluxShape shape = flux_shape(s->N1D, s->K, s->geo.elems_per_block_flux,
-                                       flags_for(s, 2, false, false) & kExtFlags, s->mixed);
+                                       flags_for(s, 2, false, false) & kExtFlags, s->mixed, sms);
     s->geo.elems_per_block = shape.epb;
     s->geo.elems_per_block_max = s->geo.elems_per_block_max_flux;
     s->base.threads = shape.threads;

@@ -39,12 +39,13 @@ struct FluxShape {
   bool split;
   int epb, threads;
 };
-inline FluxShape flux_shape(int n1d, int K, int epb_lines, bool ext, bool acc64) {
+// sms: multiprocessors of the device.
+inline FluxShape flux_shape(int n1d, int K, int epb_lines, bool ext, bool acc64, int sms) {
   const int64_t nodes = (int64_t)K * n1d * n1d;
   if (!ext && nodes < (n1d >= 5 ? 110000 : 65536))
     return {true, n1d == 2 ? 8 : n1d == 3 || n1d == 5 ? 3 : 2, 128};
   if (acc64 && n1d >= 5) epb_lines = n1d == 5 ? 5 : 6;
-  const bool wide = n1d == 3 || (acc64 && n1d == 6) || (K + epb_lines - 1) / epb_lines < 10 * 152;
+  const bool wide = n1d == 3 || (acc64 && n1d == 6) || (K + epb_lines - 1) / epb_lines < 10 * sms;
   return {false, epb_lines, wide ? 128 : 64};
 }
 
