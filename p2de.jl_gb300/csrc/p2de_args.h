@@ -97,9 +97,9 @@ struct StageArgs {
   double* ufproj;       // K x Nfp x 4: entropy-projected face states (GaussCollocation)
   double* theta;        // 3 stages x K x Nfp: entropy-projection limiting factors
   double eta;           // LimitingParameter eta (bounds of the projected face states)
-  // constants of the gas, formed once (set_gas): 1/(gamma-1), gamma (gamma-1)/4, and FP32
-  // gamma, gamma-1, 2 (gamma-1)
-  double rgm1, cws;
+  // constants of the gas, formed once (set_gas): 1/(gamma-1), (gamma-1)/2, gamma (gamma-1)/4,
+  // and FP32 gamma, gamma-1, 2 (gamma-1)
+  double rgm1, hgm1, cws;
   float gasf[3];
   // floor(log2((1 - zeta)/zeta)) (set_zeta): the quadratics' constant term is at least
   // rho (zeta rhoe) 2^kzeta; very negative when zeta is not in (0, 1)
@@ -115,6 +115,7 @@ inline void set_gas(StageArgs& a, double gamma) {
   a.gamma = gamma;
   a.gm1 = gamma - 1.0;
   a.rgm1 = 1.0 / a.gm1;
+  a.hgm1 = 0.5 * a.gm1;
   a.cws = 0.25 * (gamma * a.gm1);
   a.gasf[0] = (float)a.gamma;
   a.gasf[1] = (float)a.gm1;

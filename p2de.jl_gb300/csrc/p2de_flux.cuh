@@ -296,9 +296,10 @@ struct FluxLine {
     P.U[3] = S[3];
     const double rr = rcp(P.U[0]), hr = half(rr);
     const double hn = dmul(P.U[1], hr), ht = dmul(P.U[2], hr);
-    // p as the node phase forms it, so that the two elements at a face form the same flux bits
-    const double p = dmul(a.gm1, dfma(-0.5, dmul(dfma(S[1], S[1], dmul(S[2], S[2])), rr), S[3]));
-    line_node(P, hn, ht, half(p), dmul(a.cws, rr));
+    // p/2 as the node phase forms it, so that the two elements at a face form the same flux bits
+    // (times gm1/2, not half of times gm1: 595 us a stage against 605 on DMR 480x120)
+    const double ph = dmul(a.hgm1, dfma(-0.5, dmul(dfma(S[1], S[1], dmul(S[2], S[2])), rr), S[3]));
+    line_node(P, hn, ht, ph, dmul(a.cws, rr));
     // a boundary face's wavespeed is the own one (its mapP is itself)
     if (code != BC_INTERIOR) P.wh = own.wh;
     off = code == BC_INFLOW || code == BC_OUTFLOW || code == BC_SHOCK;
@@ -421,6 +422,7 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
   // SPLIT deals a node's logarithms to other warps (part 1: log rho; part 2: beta, from its own
   // copy of p, and log beta), each part in whole warps
   constexpr int parts = SPLIT && !F32 ? 3 : 1;
+  bool far = false;  // some state from which a flux may overflow
   const int n32 = parts == 1 ? Ke * Nq : (Ke * Nq + 31) & ~31;
   for (int v = tid; v < parts * n32; v += bs) {
     const int part = v / n32, w = v % n32;
@@ -451,9 +453,16 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
     U[3 * Nq] = En;
     const double hr = half(rr);
     const double hu = dmul(m1, hr), hv = dmul(m2, hr);
-    // a state the reference would stop on (DomainError from log or sqrt of a negative,
-    // flux_differencing.jl:49-50): density or pressure -0, negative or NaN
-    if (!positive_bits(rho) || !positive_bits(p)) atomicOr(a.status, ST_NOT_POSITIVE);
+    // rho in [2^-24, 2^24), p in [2^-40, 2^30), E < 2^30: no two-point flux of such states
+    // overflows, in FP32 either (beta in [2^-55, 2^63], |u| <= 2^27.5, so the terms of the energy
+    // flux stay below 2^108 / (gamma - 1))
+    if (!((unsigned)(__double2hiint(rho) - (999 << 20)) < (48u << 20) &&
+          (unsigned)(__double2hiint(p) - (983 << 20)) < (70u << 20) && __double2hiint(En) < (1053 << 20))) {
+      far = true;
+      // a state the reference would stop on (DomainError from log or sqrt of a negative,
+      // flux_differencing.jl:49-50): density or pressure -0, negative or NaN
+      if (!positive_bits(rho) || !positive_bits(p)) atomicOr(a.status, ST_NOT_POSITIVE);
+    }
     W[C::W_HU * Nq] = hu;
     W[C::W_HV * Nq] = hv;
     W[C::W_PH * Nq] = half(p);
@@ -478,7 +487,7 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
       }
     }
   }
-  __syncthreads();
+  const bool overflow = __syncthreads_or(far);
 
   // ---- smoothness indicator (shock_capture.jl:49-81): modal energies through inv(VDM), the
   //      Hennemann blending factor (:118-137) and the relaxed bounds' smoothness factor
@@ -1138,7 +1147,10 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
 
   // ---- limited fluxes (accumulate_f_bar_limited!, subcell.jl:841-876): phi + l dF where the
   //      face blends anything. A boundary face with dF != 0 is its own neighbour, so its
-  //      factor is final here; the others' factors multiply 0.
+  //      factor is final here; the others' factors multiply 0. Where a flux may overflow, all
+  //      faces: 0 x Inf = NaN ends the step. (DMR 480x120, FP64: 595 us a stage with the lines
+  //      looking at their high-order fluxes, 589 with the node phase looking at the states,
+  //      590 with neither.)
   for (int w = tid; w < Ke * NF; w += bs) {
     const int e = w < Ke * NI ? w / NI : (w - Ke * NI) / (NF - NI);
     const int r = w < Ke * NI ? w % NI : NI + (w - Ke * NI) % (NF - NI);
@@ -1148,20 +1160,9 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
     const double L = base[Y::O_L + f];
     double* PH = base + Y::O_PH + f;
     const double* DF = base + Y::O_DF + f;
-    bool on = !is_zero_bits(L) && (r < NI || !(is_zero_bits(DF[0]) && is_zero_bits(DF[NF]) &&
-                                               is_zero_bits(DF[2 * NF]) && is_zero_bits(DF[3 * NF])));
-    bool inf = false;  // the face's fluxes overflow: phi + l (phi_H - phi_L) also where l is 0
-#pragma unroll
-    for (int c = 0; c < 4; ++c) inf = inf || may_overflow(DF[c * NF]) || may_overflow(PH[c * NF]);
-    if (inf) {
-#pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
-        // only interior faces keep phi_H in DF (O_DF)
-        const double h = r < NI && negative(L) ? DF[c * NF] : dadd(PH[c * NF], DF[c * NF]);
-        PH[c * NF] = dfma(fabs(L), dsub(h, PH[c * NF]), PH[c * NF]);
-      }
-      on = true;
-    } else if (on) {
+    const bool on = overflow || (!is_zero_bits(L) && (r < NI || !(is_zero_bits(DF[0]) && is_zero_bits(DF[NF]) &&
+                                                                  is_zero_bits(DF[2 * NF]) && is_zero_bits(DF[3 * NF]))));
+    if (on) {
 #pragma unroll
       for (int c = 0; c < 4; ++c) PH[c * NF] = dfma(L, DF[c * NF], PH[c * NF]);
     }

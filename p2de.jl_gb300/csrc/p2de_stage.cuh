@@ -201,10 +201,11 @@ __device__ __forceinline__ bool magnitude_above(double x, double t) {
   return b > __double_as_longlong(t) && b <= 0x7ff0000000000000LL;
 }
 
-// |x| >= 2^1023, infinite or NaN: a difference with it may not be finite
-__device__ __forceinline__ bool may_overflow(double x) {
-  return (__double2hiint(x) & 0x7fffffff) >= 0x7fe00000;
-}
+// |x| >= 2^1023, infinite or NaN: a difference with it may not be finite. high_bits orders
+// magnitudes, so that one comparison serves the largest of several.
+__device__ __forceinline__ unsigned high_bits(double x) { return (unsigned)__double2hiint(x) << 1; }
+constexpr unsigned kOverflowBits = 0x7fe00000u << 1;
+__device__ __forceinline__ bool may_overflow(double x) { return high_bits(x) >= kOverflowBits; }
 
 // fluxes(Dim2) (:175-194) with 1/rho given
 __device__ __forceinline__ void fluxes_r(const Gas<double>& g, const double* U, double rr, double* fx, double* fy) {
@@ -957,6 +958,7 @@ __device__ __forceinline__ void stage_a_body(const StageArgs& a, int k0, double*
   if (tid == 0) {
     s_list[0] = 0;
     s_list[NEV * E + 1] = 0;  // the count of the bisections' list (P9)
+    s_list[NEV * E + 2] = 0;  // whether some subcell flux may overflow (P8)
   }
   for (int w = tid; w < Ke * Nq * 4; w += bs) {
     int e = w / (Nq * 4), r = w % (Nq * 4);
@@ -1868,6 +1870,7 @@ __device__ __forceinline__ void stage_a_body(const StageArgs& a, int k0, double*
     double h = base[C::O_BFH + 8 * f0 + o], lo = base[C::O_BFL + 8 * f0 + o];
     fH[fb0 * 4 + c] = h;
     fL[fb0 * 4 + c] = lo;
+    unsigned big = max(high_bits(h), high_bits(lo));
     for (int t = 1; t <= n; ++t) {
       const int q = qb0 + qs * (t - 1);
       const double wJ = wJq[2 * q];
@@ -1875,7 +1878,9 @@ __device__ __forceinline__ void stage_a_body(const StageArgs& a, int k0, double*
       lo = lo + wJ * base[C::O_RXYL + 8 * q + o];
       fH[(fb0 + fs * t) * 4 + c] = h;
       fL[(fb0 + fs * t) * 4 + c] = lo;
+      big = max(big, max(high_bits(h), high_bits(lo)));
     }
+    if (big >= kOverflowBits) s_list[NEV * E + 2] = 1;
   }
   for (int w = tid; w < Ke * Nq; w += bs) {
     int e = w / Nq, m = w % Nq;
@@ -2298,21 +2303,25 @@ __device__ __forceinline__ void stage_a_body(const StageArgs& a, int k0, double*
     __syncthreads();
   }
 
-  // ---- P12: the subcell fluxes and L before symmetrization for kernel B. A face whose fluxes
+  // ---- P12: L before symmetrization and the subcell fluxes for kernel B. A face whose fluxes
   //      overflow (FP32 terms do from 2^128 on) has the sign bit of its L set: kernel B then
-  //      forms the combination also where L is 0, whose 0 x Inf = NaN ends the step.
-  for (int w = tid; w < Ke * C::FBAR; w += bs) {
-    const int e = w / C::FBAR, r = w % C::FBAR;
-    const double v = sm[e * PE + C::O_SCR + r];
-    a.fbar[(size_t)(k0 + e) * C::FBAR + r] = v;
-    if (may_overflow(v))
-      atomicOr(reinterpret_cast<unsigned long long*>(sm + e * PE + C::O_L + r / (8 * NSF) * NSF + r / 4 % NSF),
-               0x8000000000000000ULL);
-  }
-  __syncthreads();
+  //      forms the combination also where L is 0, whose 0 x Inf = NaN ends the step. P8 has
+  //      looked whether the block has any (every face looked at here cost the mixed DMR step 1%).
+  const bool overflow = s_list[NEV * E + 2] != 0;
   for (int w = tid; w < Ke * 2 * NSF; w += bs) {
     int e = w / (2 * NSF), r = w % (2 * NSF);
-    a.Lpre[(size_t)(k0 + e) * 2 * NSF + r] = sm[e * PE + C::O_L + r];
+    double L = sm[e * PE + C::O_L + r];
+    if (overflow) {
+      const double* fb = sm + e * PE + C::O_SCR + (r / NSF * 2 * NSF + r % NSF) * 4;  // f_H, f_L NSF faces on
+      bool over = false;
+      for (int c = 0; c < 4; ++c) over = over || may_overflow(fb[c]) || may_overflow(fb[4 * NSF + c]);
+      if (over) L = __longlong_as_double(__double_as_longlong(L) | (long long)0x8000000000000000ULL);
+    }
+    a.Lpre[(size_t)(k0 + e) * 2 * NSF + r] = L;
+  }
+  for (int w = tid; w < Ke * C::FBAR; w += bs) {
+    int e = w / C::FBAR, r = w % C::FBAR;
+    a.fbar[(size_t)(k0 + e) * C::FBAR + r] = sm[e * PE + C::O_SCR + r];
   }
 }
 
