@@ -16,8 +16,10 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 BUILD = PKG / "_build"
 LIB = BUILD / "libp2de_gpu.so"
-# the benchmark's FP64/FP32 FMA-throughput probe (roofline denominator), kept out of the solver
-PROBE_SRC = CSRC / "probe" / "p2de_fma_probe.cu"
+# the benchmark's FP64/FP32 FMA-throughput probe (roofline denominator) and the point
+# arithmetic's for its tests, kept out of the solver
+PROBE_SRCS = sorted((CSRC / "probe").glob("*.cu")) + [CSRC / "p2de_tables.cpp"]
+PROBE_DEPS = PROBE_SRCS + [CSRC / "p2de_arith.cuh", CSRC / "p2de_tables.h"]
 PROBE_LIB = BUILD / "libp2de_probe.so"
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
@@ -60,17 +62,17 @@ def up_to_date() -> bool:
 
 
 def build_probe(force: bool = False, verbose: bool = False) -> Path:
-    """libp2de_probe.so: the benchmark's FMA-throughput probe, one translation unit."""
-    if not force and PROBE_LIB.exists() and PROBE_LIB.stat().st_mtime >= PROBE_SRC.stat().st_mtime:
+    """libp2de_probe.so: the benchmark's FMA-throughput probe and the tests' arithmetic probe."""
+    if not force and PROBE_LIB.exists() and all(p.stat().st_mtime <= PROBE_LIB.stat().st_mtime for p in PROBE_DEPS):
         return PROBE_LIB
     BUILD.mkdir(parents=True, exist_ok=True)
     tmp = PROBE_LIB.with_suffix(".so.tmp")
-    cmd = [_nvcc(), *NVCC_FLAGS, "-shared", str(PROBE_SRC), "-o", str(tmp)]
+    cmd = [_nvcc(), *NVCC_FLAGS, "-shared", *map(str, PROBE_SRCS), "-o", str(tmp)]
     if verbose:
         print(" ".join(cmd), flush=True)
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
-        raise RuntimeError(f"nvcc failed for {PROBE_SRC.name}:\n{r.stdout}\n{r.stderr}")
+        raise RuntimeError(f"nvcc failed for {PROBE_LIB.name}:\n{r.stdout}\n{r.stderr}")
     os.replace(tmp, PROBE_LIB)
     return PROBE_LIB
 

@@ -135,11 +135,11 @@ __device__ __forceinline__ double log_fast(double x, const Tab& op) {
   return hi + (p + lo);
 }
 
-// exp(h + l) for |h| < 700 and |l| below an ulp of h, by the table-driven method of P. T. P. Tang
+// exp(h + l) for |h| < 700 and |l| < 0.001, by the table-driven method of P. T. P. Tang
 // ("Table-driven implementation of the exponential function in IEEE floating-point arithmetic",
 // ACM TOMS 15(2), 1989): h + l = (128 e + j) log 2 / 128 + r with |r| < 0.0028, the result is
 // 2^e (T_j + T_j (exp r - 1)) with T_j = 2^(j/128) in two parts and the Taylor polynomial of
-// exp r - 1 to r^5 (the next term is below 2^-60).
+// exp r - 1 to r^5 (the next term is below 2^-57.6 with the largest l, 2^-60 with none).
 template <class Tab>
 __device__ __forceinline__ double exp_parts(double h, double l, const Tab& op) {
   const double t = __fma_rn(h, op.exp_inv, 0x1.8p52);
@@ -163,13 +163,16 @@ __device__ __forceinline__ double exp_fast(double x, const Tab& op) {
 }
 
 // x^y as exp(y log x), with log x in two parts from the table of log_fast (its r = (m - F)/F is
-// accurate to 2^-61, the parts' sum to about 2^-60), the product in two parts, and exp_parts:
-// about 0.51 ulp, 33 FP64 operations against 86 for pow(). x positive and normal with
-// |y log x| < 700; other arguments take pow().
+// accurate to 2^-60.5, and so are the parts), the product in two parts, and exp_parts:
+// 0.5 + |y| 2^-7.5 ulp, 33 FP64 operations against 86 for pow(), which takes 1.3 ulp. x positive
+// and normal with |y log x| < 700, |y| < 128 (where |y| 2^-18 of the second part stays well
+// within exp_parts' polynomial, and the error below pow's); other arguments take pow().
 template <class Tab>
 __device__ __forceinline__ double pow_fast(double x, double y, const Tab& op) {
   const long long b = __double_as_longlong(x);
-  if ((unsigned long long)(b - 0x0010000000000000LL) >= 0x7fe0000000000000ULL) return pow(x, y);
+  if ((unsigned long long)(b - 0x0010000000000000LL) >= 0x7fe0000000000000ULL ||
+      (unsigned)(__double2hiint(y) & 0x7fffffff) >= 0x40600000u)
+    return pow(x, y);
   long long k = (b >> 52) - 1023;
   long long mb = (b & 0x000fffffffffffffLL) | 0x3ff0000000000000LL;
   if (((mb >> 44) & 0xff) >= 106) {
@@ -183,7 +186,7 @@ __device__ __forceinline__ double pow_fast(double x, double y, const Tab& op) {
   const double* T = op.logtab[j - kLogTabLo];
   const double r = __dmul_rn(__dsub_rn(__longlong_as_double(mb), F), T[0]);
   const double kd = __dsub_rn(__longlong_as_double(0x4338000000000000LL + k), 0x1.8p52);
-  const double hi = __fma_rn(kd, op.ln2_hi, T[1]);
+  const double hi = __fma_rn(kd, op.ln2_hi, T[3]);          // exact
   const double s = __dadd_rn(hi, r);                        // |hi| >= |r| or hi = 0
   const double e = __dadd_rn(__dsub_rn(hi, s), r);          // its rounding
   double q = __fma_rn(r, -1.0 / 6.0, 1.0 / 5.0);
@@ -191,7 +194,7 @@ __device__ __forceinline__ double pow_fast(double x, double y, const Tab& op) {
   q = __fma_rn(q, r, 1.0 / 3.0);
   const double r2 = __dmul_rn(r, r);
   const double p = __fma_rn(__dmul_rn(r2, r), q, __dmul_rn(-0.5, r2));
-  const double lo = __dadd_rn(__dadd_rn(p, e), __fma_rn(kd, op.ln2_lo, T[2]));
+  const double lo = __dadd_rn(__dadd_rn(p, e), __fma_rn(kd, op.ln2_lo, T[4]));
   const double h = __dmul_rn(y, s);
   const double l = __fma_rn(y, lo, __fma_rn(y, s, -h));
   if ((unsigned)(__double2hiint(h) & 0x7fffffff) >= 0x4085e000u) return pow(x, y);

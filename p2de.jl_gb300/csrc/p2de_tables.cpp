@@ -190,7 +190,7 @@ static void split_hi_lo(long double v, int bits, double* hi, double* lo) {
 // The tables of log_fast and exp_fast, the same for every solve: formed once per process, as
 // the long double functions run in software on Arm (about 130 us of a solver's creation)
 struct FunctionTables {
-  double logtab[kLogTabN][3];
+  double logtab[kLogTabN][5];
   double ln2_hi, ln2_lo;
   double exptab[128][2];
   double exp_inv, exp_hi, exp_lo;
@@ -198,7 +198,10 @@ struct FunctionTables {
     for (int i = 0; i < kLogTabN; ++i) {
       const int j = kLogTabLo + i;
       logtab[i][0] = 256.0 / j;
-      split_hi_lo(std::log((long double)j / 256.0L), 41, &logtab[i][1], &logtab[i][2]);
+      const long double v = std::log((long double)j / 256.0L);
+      split_hi_lo(v, 41, &logtab[i][1], &logtab[i][2]);
+      logtab[i][3] = (double)std::ldexp(std::trunc(std::ldexp(v, 42)), -42);
+      logtab[i][4] = (double)(v - (long double)logtab[i][3]);
     }
     split_hi_lo(std::log(2.0L), 42, &ln2_hi, &ln2_lo);
     for (int j = 0; j < 128; ++j) {

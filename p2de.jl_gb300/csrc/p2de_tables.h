@@ -65,8 +65,10 @@ struct OpTable {
   // r=-1, r=+1, s=-1, s=+1 in order): Vf[f, m] / wq[m] (init.jl:171-172)
   double liftf[kMaxNq][4];
   // log_fast: per j, 1/F_j, log F_j to 41 significant bits and the rest of log F_j; log 2 in
-  // the same two parts (42 significant bits, so that k log2_hi is exact for |k| < 2048)
-  double logtab[kLogTabN][3];
+  // the same two parts (42 significant bits, so that k log2_hi is exact for |k| < 2048); for
+  // pow_fast log F once more as a multiple of 2^-42, the last bit of log2_hi, and the rest, so
+  // that k log2_hi + log F is exact too
+  double logtab[kLogTabN][5];
   double ln2_hi, ln2_lo;
   // exp_fast: 2^(j/128) in two parts, 128/log 2, log 2/128 to 35 bits and the rest
   double exptab[128][2];
@@ -95,7 +97,7 @@ struct LineOps {
   int8_t pi[kLineMaxPairs], pj[kLineMaxPairs];  // its nonzero pairs i > j, j outer (init.jl:188-195)
   double MinvVhT[kMaxN1D * kLineMaxNh];   // M \ Vh' = (1/wq) [I, Vf'], column-major Nq x Nh
   double VDMinv[kMaxN1D * kMaxN1D];       // inv(VDM) of the orthonormal Legendre modes, row-major
-  double logtab[kLogTabN][3];             // log_fast, as in OpTable
+  double logtab[kLogTabN][5];             // log_fast, as in OpTable
   double ln2_hi, ln2_lo;
   // exp_fast: 2^(j/128) in two parts, 128/log 2, log 2/128 to 35 bits and the rest
   double exptab[128][2];
