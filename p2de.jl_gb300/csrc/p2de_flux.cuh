@@ -63,12 +63,13 @@ struct FluxCfg {
   static constexpr int O_U = O_C + 6 * n;       // 4 Nq: state
   static constexpr int O_W = O_U + 4 * Nq;      // 12 Nq (14 Nq EXT): node data, see W_*
   // W before the line phase: u/2, v/2, u, v, rho/p, log rho, log(rho/p), p/2, gamma gm1/(4 rho)
-  // (FP32: planes 2-3 hold rho, u, v, beta as floats); indicator and modal energies 9, 10.
+  // (FP32 pairs: planes 4-5, W_F32, hold rho, u, v, beta as floats); indicator and modal
+  // energies 9, 10.
   // After it: uL (0-3), zeta rhoe, Lrho, Urho, phi threshold, the quadratics' c; EXT: bound
   // evaluations 10-13.
   // In the cell-entropy phase: its scratch.
   static constexpr int W_HU = 0, W_HV = 1, W_U = 2, W_V = 3, W_BETA = 4, W_LR = 5, W_LB = 6, W_PH = 7, W_CRR = 8,
-                       W_IND = 9, W_EN = 10;
+                       W_IND = 9, W_EN = 10, W_F32 = 4;
   static constexpr int W_UL = 0, W_LRHOE = 4, W_LRHO = 5, W_URHO = 6, W_THR = 7, W_QC = 8, W_EV = 10;
   static constexpr int NPH = NL * PPL;
   template <bool EXT, bool SPLIT = false>
@@ -348,7 +349,7 @@ struct FluxLine {
       pstate(mj, qj);
       fS_line(a.rgm1, qj, qi, &F[0], &F[2], &F[1], &F[3]);
     } else {
-      const float* Wf = reinterpret_cast<const float*>(base + C::O_W + 4 * Nq);
+      const float* Wf = reinterpret_cast<const float*>(base + C::O_W + C::W_F32 * Nq);
       const float UJ[4] = {Wf[mj], Wf[Nq + mj], Wf[2 * Nq + mj], Wf[3 * Nq + mj]};
       const float UI[4] = {Wf[mi], Wf[Nq + mi], Wf[2 * Nq + mi], Wf[3 * Nq + mi]};
       const float c = op.hpcf[(ax * n + l) * C::PPL + i * (i - 1) / 2 + j];
@@ -470,7 +471,7 @@ __device__ __forceinline__ void flux_a_body(const StageArgs& a, int k0, double* 
     if (EXT && (flags & F_RELAXED) || (flags & F_SHOCK)) W[C::W_IND * Nq] = dmul(rho, p);  // shock_capture.jl:92-103
     if (F32) {
       // FP32 (rho, u, v, beta), converted once per node
-      float* Wf = reinterpret_cast<float*>(base + C::O_W + 4 * Nq) + m;
+      float* Wf = reinterpret_cast<float*>(base + C::O_W + C::W_F32 * Nq) + m;
       const float rf = (float)rho;
       Wf[0] = rf;
       Wf[Nq] = 2.0f * (float)hu;

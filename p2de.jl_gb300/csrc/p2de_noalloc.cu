@@ -41,7 +41,9 @@ constexpr size_t H_DATA = H_TABLE + kTableDoubles;
 // doubles of solve data a call may use: the published budget less the header and the table's
 // first size, so that the largest accepted K does not change as the table grows (the array
 // holds the growth on top)
-constexpr size_t kDataDoubles = kScratchDoubles - H_TABLE - 2976;
+constexpr size_t kFirstTableDoubles = 2976;
+constexpr size_t kDataDoubles = kScratchDoubles - H_TABLE - kFirstTableDoubles;
+static_assert(kTableDoubles >= kFirstTableDoubles, "the array holds the table's growth");
 static __device__ __align__(256) double g_noalloc_scratch[H_DATA + kDataDoubles];
 
 struct DeviceState {

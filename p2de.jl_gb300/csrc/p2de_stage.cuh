@@ -110,7 +110,8 @@ struct Cfg {
   static constexpr int O_PF = O_UF + 4 * Nfp;       // 6 Nfp
   static constexpr int O_TH = O_PF + 6 * Nfp;       // Nfp
   static constexpr int O_QFF = O_TH + Nfp;          // 8 Nfp
-  static constexpr int O_FPT = O_QFF + 8 * Nfp;     // 8 Nfp n: pair (face f, line node a) at f n + a
+  static constexpr int O_FPT = O_QFF + 8 * Nfp;     // 8 Nfp n: pair (face f, line node a) at f n + a; of
+                                                    // axis-aligned elements only the face's own axis
   static constexpr int PER_ELEM_G = (O_FPT + 8 * Nfp * n + 1) & ~1;
   static constexpr size_t smem_g(int e) { return sizeof(double) * PER_ELEM_G * e + sizeof(int) * (NEV * e + 4); }
   static constexpr int E_G = (64 / Nq) > 0 ? (64 / Nq) : 1;
