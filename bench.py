@@ -43,11 +43,14 @@ sys.path.insert(0, str(ROOT))
 METRIC = "DOF-stage updates/s, 2D Euler N=3; served solves/s + p99 vs plain, same L1 err"
 UNIT = "DOF-stage updates/s"
 
-# stage kernel A on this workload from one ncu capture
-# (profiles/k_flux_a_dmr480x120_n3.md): DRAM traffic per launch
-# (dram__bytes_read.sum + dram__bytes_write.sum) and the FP64 pipe's busy fraction
-KERNEL_A_TRAFFIC_BYTES = 49.3e6
-KERNEL_A_FP64_PIPE_BUSY = 0.835
+# stage kernel A on the 480x120 N=3 mesh from one ncu capture
+# (profiles/k_flux_a_dmr480x120_n3.md), by (basis, precision): DRAM traffic per launch
+# (dram__bytes_read.sum + dram__bytes_write.sum) and the FP64 pipe's busy fraction; the modes
+# not captured print null
+KERNEL_A_NCU = {
+    ("lobatto", "fp64"): {"traffic": 49.3e6, "fp64_pipe_busy_ncu": 0.835},
+    ("lobatto", "mixed"): {"traffic": 147.5e6, "fp64_pipe_busy_ncu": 0.645},
+}
 
 
 def fma_probe_library():
@@ -723,7 +726,10 @@ def main():
     quad_per_launch = cnt[0] / (3 * prof_steps)
     # the workload runs in flux form but for FP32 accumulation and Gauss nodes
     flux = args.precision != "mixed" and args.basis == "lobatto"
-    flops_a = (roofline.flux_form_flops if flux else roofline.stage_a_flops)(param.N, desc.K, quad_per_launch)
+    if flux:
+        flops_a = roofline.flux_form_flops(param.N, desc.K, quad_per_launch, args.precision != "fp64")
+    else:
+        flops_a = roofline.stage_a_flops(param.N, desc.K, quad_per_launch, args.precision, param.reference_semantics)
     peak = c_double()
     probe = fma_probe_library()
     rc = probe.p2de_probe_fma_peak(local, 1, byref(peak))
@@ -799,7 +805,8 @@ def main():
         cpu = None
         if not args.no_cpu_baseline:
             cpu = cpu_baseline(desc, U0, nodes)
-        bytes_ab = roofline.stage_bytes(param.N, desc.K)
+        bytes_ab = roofline.stage_bytes(param.N, desc.K, flux)
+        ncu = KERNEL_A_NCU.get((args.basis, args.precision)) if args.workload == "dmr" and not args.mesh else None
         line = {
             "metric": METRIC,
             "value": value,
@@ -819,7 +826,7 @@ def main():
                 "nodes": nodes,
                 "precision": args.precision,
                 "parallelism": f"replicas x{world}" if world > 1 else "single solve",
-                "l2": "working set per step > L2 (stage data ~%.0f MB per launch)" % (bytes_ab["stage_a"] / 1e6),
+                "l2": "no flush: a step's arrays are %.0f MB, the L2 129 MB" % (roofline.step_bytes(param.N, desc.K) / 1e6),
                 "timing": "CUDA-graph replay of whole steps, CUDA events on the launching stream",
                 "elements_per_block": epb,
                 "elements_per_block_source": "default" if args.no_autotune else f"autotuned (default {epb_default})",
@@ -842,13 +849,14 @@ def main():
                 "peak": peak.value,
                 "unit": "TFLOP/s",
                 "frac": achieved / peak.value,
-                "traffic": KERNEL_A_TRAFFIC_BYTES,
-                "fp64_pipe_busy_ncu": KERNEL_A_FP64_PIPE_BUSY,
+                "traffic": ncu and ncu["traffic"],
+                "fp64_pipe_busy_ncu": ncu and ncu["fp64_pipe_busy_ncu"],
                 "algorithmic_flops_per_launch": flops_a,
                 "quad_solves_per_launch": quad_per_launch,
                 "ms_per_launch": kms[0],
                 "ms_per_launch_stage_b": kms[1],
-                "stage_b_hbm_gbs": bytes_ab["stage_b"] / (kms[1] * 1e-3) / 1e9,
+                # of algorithmic bytes; rhsU and the factors come from the L2 where kernel A left them there
+                "stage_b_gbs": bytes_ab["stage_b"] / (kms[1] * 1e-3) / 1e9,
                 "peak_source": "libp2de_probe.so p2de_probe_fma_peak: FP64 FMA chains on this GPU in this run (MEASURED_PEAKS.json has no FP64 figure)",
             },
             "min_rho_rhoe_last_step": [float(mins[4]), float(mins[5])],
