@@ -79,3 +79,31 @@ def test_large_boundary_fluxes_with_a_finite_difference_stay_finite(rho):
     assert np.isfinite(g.get_field(abi.FIELD_F_BAR_L)).all() and np.isfinite(g.get_field(abi.FIELD_F_BAR_H)).all()
     assert np.isfinite(g.get_field(abi.FIELD_RHSU)).all()
     g.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed-acc64"])
+@pytest.mark.parametrize("N", [1, 2, 3, 4, 5])
+def test_states_from_which_fluxes_may_overflow_give_the_same_bits(N, precision):
+    """Blocks with a density outside [2^-24, 2^24), a pressure outside [2^-40, 2^30) or an energy
+    from 2^30 on combine all their faces. Under the reference's reading the factors are 0, so
+    rhsU is the low-order one, which scales exactly with powers of two from states inside the
+    ranges: density by 2^a, velocity by 2^c."""
+    param, md, bc, desc, U0 = setup(problems.riemann2d, N=N, Kx=5, Ky=4, bound=PositivityBound(), precision=precision)
+    rng = np.random.default_rng(N)
+    shape = U0.shape[:-1]
+    rho, p = 0.5 + rng.random(shape), 0.5 + rng.random(shape)
+    u, v = rng.standard_normal((2, *shape))
+    U = np.stack([rho, rho * u, rho * v, p / 0.4 + 0.5 * rho * (u * u + v * v)], axis=-1)
+
+    def rhs(a, c):
+        g = S.Solver(param, md, desc)
+        g.set_Uq(U * np.exp2([a, a + c, a + c, a + 2 * c]))
+        S.rhs_bang(None, g, None, p2de.TimeParam(0.0, 2.0 ** (-14 - c), 2))
+        out = g.get_field(abi.FIELD_RHSU).reshape(U.shape)
+        g.close()
+        return out * np.exp2(-np.array([a + c, a + 2.0 * c, a + 2 * c, a + 3 * c]))
+
+    want = rhs(0, 0)
+    assert np.isfinite(want).all()
+    for a, c in ((25, 0), (-26, 0), (0, 16), (0, -22), (10, 5)):  # the last one inside the ranges
+        np.testing.assert_array_equal(rhs(a, c), want, err_msg=f"{a} {c}")
