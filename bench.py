@@ -48,7 +48,7 @@ UNIT = "DOF-stage updates/s"
 # (dram__bytes_read.sum + dram__bytes_write.sum) and the FP64 pipe's busy fraction; the modes
 # not captured print null
 KERNEL_A_NCU = {
-    ("lobatto", "fp64"): {"traffic": 49.3e6, "fp64_pipe_busy_ncu": 0.835},
+    ("lobatto", "fp64"): {"traffic": 48.8e6, "fp64_pipe_busy_ncu": 0.835},
     ("lobatto", "mixed"): {"traffic": 147.5e6, "fp64_pipe_busy_ncu": 0.645},
 }
 
